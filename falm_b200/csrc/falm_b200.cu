@@ -35,6 +35,7 @@
 #include "plane3_tma.cuh"
 #include "falm_io.cuh"
 #include "sor_rb_tma.cuh"
+#include "pc_mv.cuh"
 #include "adjoint.cuh"
 #include "rmcp.cuh"
 #include <cudaTypedefs.h>

@@ -132,6 +132,7 @@ struct falm_ctx {
     void *op_mem;
     fb::PoissonTables<double> pt64;
     fb::PoissonTables<float> pt32;
+    int zrun0, zrun1;                       // longest run of planes [zrun0, zrun1) with equal z coefficients
     const void *A_explicit;                 // caller-owned 7-column matrix or NULL
     // BC
     int bc_kind;

@@ -378,6 +378,59 @@ bool pc_first_in_xp(const falm_ctx *ctx) {
     return (passes & 1) != 0;
 }
 
+// Whether the solver's iterations run as fused half iterations (pc_mv.cuh):
+// the drivers' preconditioner (red-black SOR, two sweeps) on the table operator.
+bool pc_half_ok(const falm_ctx *ctx) {
+    return ctx->pc_type == FALM_LS_SOR && ctx->pc_maxit == 2 && !ctx->A_explicit && !ctx->no_tma && !ctx->sor_v1;
+}
+
+// whether the interior's cells can be accessed in aligned pairs from the first
+// one of a row: rows and bases (of the caller's vectors; the context's are
+// 256-byte aligned) on multiples of two cells, an even interior width
+template <typename T>
+bool pairs_ok(const falm_ctx *ctx, const T *a, const T *b) {
+    const Geom &g = ctx->geo;
+    return ((g.gc | g.sx | g.nx) & 1) == 0 && (((uintptr_t)a | (uintptr_t)b) % (2 * sizeof(T))) == 0;
+}
+
+// z planes per CTA of a half iteration: the chunk that minimises waves x
+// (planes + the eight of the pipeline's fill + about six for the start and the
+// reduction); one CTA is resident per SM
+template <typename T>
+int pc_chunk(const falm_ctx *ctx, long long tiles, int nz) {
+    int best = 1;
+    long long best_t = -1;
+    for (int kc = std::min(nz, PCTile<T>::KMAX); kc >= std::min(nz, 2); kc--) {
+        const long long ctas = tiles * ((nz + kc - 1) / kc);
+        if (ctas > ctx->red.maxBlocks) break;
+        const long long t = ((ctas + ctx->sm_count - 1) / ctx->sm_count) * (kc + 2 * PCTile<T>::H + 6);
+        if (best_t < 0 || t < best_t) { best_t = t; best = kc; }
+    }
+    return best;
+}
+
+// one half iteration: MODE 0 the p half (z = pp), 1 the s half (z = ss)
+template <typename T, int MODE>
+int pc_mv_launch(falm_ctx *ctx, cudaStream_t st, const T *r, T *z) {
+    using L = PCTile<T>;
+    const Geom &g = ctx->geo;
+    PCVec<T> v;
+    v.rr = (const T *)ctx->w_rr;
+    v.r = r;
+    v.a0 = (T *)ctx->w_p; v.b0 = (T *)ctx->w_q;
+    v.a1 = (T *)ctx->w_s; v.b1 = (T *)ctx->w_t;
+    v.z = z;
+    auto kern = pairs_ok(ctx, r, r) ? k_pc_mv<T, MODE, true> : k_pc_mv<T, MODE, false>;
+    constexpr int smem = L::template smem<MODE == 0 ? 3 : 2>();
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int bx = L::tiles_x(g.nx), by = L::tiles_y(g.ny);
+    const int kc = pc_chunk<T>(ctx, (long long)bx * by, g.nz);
+    const dim3 grid(bx, by, (g.nz + kc - 1) / kc);
+    LAUNCH(MODE == 0 ? FALM_K_MV_DOT1 : FALM_K_MV_DOT2, st,
+           kern<<<grid, L::NT, smem, st>>>(g, kc, op7<T>(ctx).t, v, (T)ctx->pc_relax, ctx->zrun0, ctx->zrun1, ctx->red, ctx->scal));
+    return FALM_OK;
+}
+
 // ring depth of the multi-field plane stream: keep >= 2 planes in flight and
 // at least two CTAs per SM
 template <typename T, int NF> struct P3Conf { static constexpr int NS = NF > 1 ? 4 : 6; };

@@ -96,6 +96,13 @@ int build_poisson(falm_ctx *ctx, int kind) {
     ctx->pt64.scale = scale; ctx->pt32.scale = (float)scale;
     ctx->pt64.koff = ctx->pt32.koff = g.koff;
     ctx->maxdiag = maxdiag;
+    // the longest run of interior planes with the same z coefficients (all but
+    // the wall planes on uniform spacing)
+    ctx->zrun0 = ctx->zrun1 = g.gc;
+    for (int a = g.gc, b; a < g.sz - g.gc; a = b) {
+        for (b = a + 1; b < g.sz - g.gc && up[2][b] == up[2][a] && um[2][b] == um[2][a];) b++;
+        if (b - a > ctx->zrun1 - ctx->zrun0) { ctx->zrun0 = a; ctx->zrun1 = b; }
+    }
     ctx->op_ready = 1;
     ctx->bc_kind_op = kind;
     // the coefficient of cell q towards q+1 equals that of q+1 towards q on every

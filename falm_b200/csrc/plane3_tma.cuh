@@ -396,7 +396,7 @@ struct UtoUUResBody {
             const double rv = (double)bv - ax;
             const T rt = (T)rv;
             rr[c] = rt;
-            pp[c] = pc_first<T>(pc_type, i, j, k + op.t.koff, rt, ac, pc_omega);
+            if (pp) pp[c] = pc_first<T>(pc_type, i, j, k + op.t.koff, rt, ac, pc_omega);
             acc[0] += rv * rv;
             acc[1] += (double)rt * (double)rt;
         }

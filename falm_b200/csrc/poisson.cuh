@@ -433,37 +433,48 @@ __global__ void __launch_bounds__(kRowThreads) k_mv_dot2(Geom g, Region3 R, Op7<
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kRowThreads) k_bicg_xr(Geom g, Region3 R, T *__restrict__ x, const T *__restrict__ pp,
-    const T *__restrict__ ss, T *__restrict__ r, const T *__restrict__ s, const T *__restrict__ t, const T *__restrict__ rr,
-    RedWork rw, SolverScalars *sc) {
+// x += alpha pp + omega ss; r = s - omega t; ||r||, the next rho.  s and t of an
+// odd iteration may lie in other vectors than an even one's (PCVec).  W: cells
+// per access, 2 where rows and bases allow pairs.
+template <typename T, int W>
+__global__ void __launch_bounds__(kRowThreads) k_bicg_xr(Geom g, Region3 R, T *x, const T *pp, const T *ss, T *r, const T *s0, const T *t0,
+                                                         const T *s1, const T *t1, const T *rr, RedWork rw, SolverScalars *sc) {
     if (sc->done) return;
+    const bool odd = sc->it & 1;
+    const T *s = odd ? s1 : s0, *t = odd ? t1 : t0;
     const T alpha = (T)sc->alpha, omega = (T)sc->omega;
+    constexpr int U = kRowILP / W;   // accesses per operand in flight
+    struct alignas(W * sizeof(T)) V { T v[W]; };
     double acc[2] = {0.0, 0.0};
     FB_FOR_ROWS(R, j, k) {
         const long long c0 = g.id(0, j, k);
-        for (int ib = R.i0 + (threadIdx.x & 31); ib < R.i1; ib += 32 * kRowILP) {
-            T xv[kRowILP], ppv[kRowILP], ssv[kRowILP], sv[kRowILP], tv[kRowILP], rrv[kRowILP];
+        for (int ib = R.i0 + W * (threadIdx.x & 31); ib < R.i1; ib += 32 * W * U) {
+            V xv[U], ppv[U], ssv[U], sv[U], tv[U], rrv[U];
 #pragma unroll
-            for (int u = 0; u < kRowILP; u++) {
-                const int i = ib + 32 * u;
-                xv[u] = ppv[u] = ssv[u] = sv[u] = tv[u] = rrv[u] = T(0);
+            for (int u = 0; u < U; u++) {
+                const int i = ib + 32 * W * u;
                 if (i < R.i1) {
                     const long long c = c0 + i;
-                    xv[u] = x[c]; ppv[u] = pp[c]; ssv[u] = ss[c]; sv[u] = s[c]; tv[u] = t[c]; rrv[u] = rr[c];
+                    xv[u] = *(const V *)(x + c); ppv[u] = *(const V *)(pp + c); ssv[u] = *(const V *)(ss + c);
+                    sv[u] = *(const V *)(s + c); tv[u] = *(const V *)(t + c); rrv[u] = *(const V *)(rr + c);
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kRowILP; u++) {
-                const int i = ib + 32 * u;
+            for (int u = 0; u < U; u++) {
+                const int i = ib + 32 * W * u;
                 if (i < R.i1) {
                     const long long c = c0 + i;
-                    x[c] = xv[u] + (alpha * ppv[u] + omega * ssv[u]);      // src/dev/FalmEqDevCall.cu:307
-                    const T rv = sv[u] - omega * tv[u];                    // :330
-                    r[c] = rv;
-                    const double rd = to_d(rv);
-                    acc[0] += rd * rd;
-                    acc[1] += rd * to_d(rrv[u]);
+                    V rv;
+#pragma unroll
+                    for (int e = 0; e < W; e++) {
+                        xv[u].v[e] = xv[u].v[e] + (alpha * ppv[u].v[e] + omega * ssv[u].v[e]);      // src/dev/FalmEqDevCall.cu:307
+                        rv.v[e] = sv[u].v[e] - omega * tv[u].v[e];                                  // :330
+                        const double rd = to_d(rv.v[e]);
+                        acc[0] += rd * rd;
+                        acc[1] += rd * to_d(rrv[u].v[e]);
+                    }
+                    *(V *)(x + c) = xv[u];
+                    *(V *)(r + c) = rv;
                 }
             }
         }

@@ -280,7 +280,6 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
     const Region3 R = interior(g);
     const int grid = row_grid(ctx, R);
     const int grid_p = row_grid_wave(ctx, R, k_bicg_p<T>), grid_s = row_grid_wave(ctx, R, k_bicg_s<T>);
-    const int grid_xr = row_grid_wave(ctx, R, k_bicg_xr<T>);
     const Op7<T> op = op7<T>(ctx);
     T *rr = (T *)ctx->w_rr, *p = (T *)ctx->w_p, *q = (T *)ctx->w_q, *s = (T *)ctx->w_s, *pp = (T *)ctx->w_pp;
     T *ss = (T *)ctx->w_ss, *t = (T *)ctx->w_t, *xp = (T *)ctx->w_xp;
@@ -303,7 +302,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
     // the stream of the iteration kernels: st, or the capture stream while a
     // device-side loop (CUDA graph) is recorded
     cudaStream_t ist = st;
-    const bool first_xp = pc_first_in_xp<T>(ctx);
+    const bool first_xp = pc_first_in_xp<T>(ctx), half = pc_half_ok(ctx);
     auto first_target = [&](T *z) -> T * { return first_xp ? xp : z; };
     // launch the remaining sweeps of one preconditioner application z ~ A^-1 v
     // (the first, pointwise sweep wrote first_target(z)); the temporally blocked
@@ -348,7 +347,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
             s7 = s7_launch<T, 1>(ctx, FALM_K_RES, ist, x, ResBody<T, true>{op, b, nullptr, nullptr, sc, 1});
         } else {
             ResBody<T> body{op, b, nullptr, rr, sc, 0};
-            body.pp = first_target(pp); body.pc_type = pct; body.pc_omega = pcw;
+            body.pp = half ? nullptr : first_target(pp); body.pc_type = pct; body.pc_omega = pcw;
             s7 = s7_launch<T, 2>(ctx, FALM_K_RES, ist, x, body);
         }
         if (s7 < 0) return -s7;
@@ -363,6 +362,13 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         CK(cudaMemcpyAsync(&sc->it, itmax, sizeof(itmax), cudaMemcpyHostToDevice, st));
         return FALM_OK;
     };
+    // the x and r update, s and t in s0, t0 at even iterations and in s1, t1 at odd ones
+    auto bicg_xr = [&](const T *s0, const T *t0, const T *s1, const T *t1) -> int {
+        const auto k2 = k_bicg_xr<T, 2>, k1 = k_bicg_xr<T, 1>;
+        const auto kern = pairs_ok(ctx, x, r) ? k2 : k1;
+        LAUNCH(FALM_K_BICG_XR, ist, kern<<<row_grid_wave(ctx, R, kern), kRowThreads, 0, ist>>>(g, R, x, pp, ss, r, s0, t0, s1, t1, rr, ctx->red, sc));
+        return FALM_OK;
+    };
     // the kernels of iteration itp of the pass (2 stands for every later
     // one): r equals rr until the first k_bicg_xr, and the first
     // iteration's p equals r, so it reads rr in their place
@@ -371,6 +377,12 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         T *pout = itp == 0 ? nullptr : p;
         const T *pin = itp == 1 ? rr : p, *pv = itp == 0 ? rr : p;
         int erc;
+        if (half) {   // the vectors of an iteration follow its parity on the device (PCVec)
+            if ((erc = pc_mv_launch<T, 0>(ctx, ist, r, pp))) return erc;
+            if ((erc = pc_mv_launch<T, 1>(ctx, ist, r, ss))) return erc;
+            if ((erc = bicg_xr(s, t, p, q))) return erc;
+            return FALM_OK;
+        }
         if (!(itp == 0 && pp_ready))
             LAUNCH(FALM_K_BICG_P, ist, k_bicg_p<T><<<grid_p, kRowThreads, 0, ist>>>(g, R, op, pout, pin, q, rin, first_target(pp), pct, pcw, sc));
         if ((erc = precondition_rest(pp, pv))) return erc;
@@ -380,7 +392,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         if ((erc = precondition_rest(ss, s))) return erc;
         S7_OR(FALM_K_MV_DOT2, ist, T, 2, ss, (MvDot2Body<T>{op, t, s, sc}),
               (k_mv_dot2<T><<<grid, kRowThreads, 0, ist>>>(g, R, op, ss, t, s, ctx->red, sc)));
-        LAUNCH(FALM_K_BICG_XR, ist, k_bicg_xr<T><<<grid_xr, kRowThreads, 0, ist>>>(g, R, x, pp, ss, r, s, t, rr, ctx->red, sc));
+        if ((erc = bicg_xr(s, t, s, t))) return erc;
         return FALM_OK;
     };
     if (rec) {

@@ -195,18 +195,19 @@ int step_pre_t(falm_ctx *ctx, const falm_fields *f, double dt, double t, cudaStr
             } else if ((rc = solver_init(ctx, st))) {
                 return rc;
             }
-            T *ppt = pc_first_in_xp<T>(ctx) ? (T *)ctx->w_xp : (T *)ctx->w_pp;
+            const Op7<T> op = op7<T>(ctx);
+            T *ppt = pc_half_ok(ctx) ? nullptr : (pc_first_in_xp<T>(ctx) ? (T *)ctx->w_xp : (T *)ctx->w_pp);
             const void *const fp[2] = {ua, p};
             const int nc[2] = {3, 1};
             int s3;
             if (chan)
                 s3 = p3_launch<T, 2, 2>(ctx, FALM_K_UTOUU_RHS, st, R, 1, fp, nc,
                                         UtoUUResBody<T, false>{UtoUUBody<T, true, false>{g, mview<T>(ctx), uu, rhs, scale}, mview<T>(ctx),
-                                                               op7<T>(ctx), (T *)ctx->w_rr, ppt, ctx->pc_type, (T)ctx->pc_relax, ctx->scal});
+                                                               op, (T *)ctx->w_rr, ppt, ctx->pc_type, (T)ctx->pc_relax, ctx->scal});
             else
                 s3 = p3_launch<T, 2, 2>(ctx, FALM_K_UTOUU_RHS, st, R, 1, fp, nc,
                                         UtoUUResBody<T, true>{UtoUUBody<T, true, true>{g, mview<T>(ctx), uu, rhs, scale}, mview<T>(ctx),
-                                                              op7<T>(ctx), (T *)ctx->w_rr, ppt, ctx->pc_type, (T)ctx->pc_relax, ctx->scal});
+                                                              op, (T *)ctx->w_rr, ppt, ctx->pc_type, (T)ctx->pc_relax, ctx->scal});
             if (s3 < 0) return -s3;
             fused_res = s3 == 1;
         }

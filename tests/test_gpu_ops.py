@@ -236,6 +236,41 @@ def test_blocked_sor_tiles_agree(lib_built, monkeypatch, shape, precision):
     np.testing.assert_array_equal(outs[0], outs[1])
 
 
+HALF_SHAPES = [(3, 2, 2), (40, 20, 3), (57, 25, 12), (64, 32, 1), (65, 24, 9), (66, 33, 30), (120, 56, 5), (121, 41, 17), (180, 63, 11)]
+
+
+@pytest.mark.parametrize("stretch", [1.0, 1.02])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shape", HALF_SHAPES)
+def test_half_iterations_match_separate_kernels(lib_built, monkeypatch, shape, precision, stretch):
+    """The fused half iterations (tiles of 64 x 32 or 64 x 24 cells that own 56 x 24
+    or 56 x 16, up to the walls where they touch them; pairs or single cells; regular
+    and general z coefficients) against the row kernels in FP64, around the tile
+    sizes and at odd widths.  FP64: three iterations to rounding, 1e-12 over the
+    growth of three iterations on these grids (below 50).  Mixed: two iterations a
+    pass from the same FP32 data, FP32 rounding (6e-8) over the same growth and five
+    passes."""
+    nx, ny, nz = shape
+    case = cases.small_channel(40, 24, 24, intensity=0.0)
+    case.grid = cases.uniform_grid(nx, ny, nz, 0.05) if stretch == 1.0 else cases.stretched_grid(nx, ny, nz, 0.05, stretch)
+    case.alm = None
+    case.pc, case.tol, case.maxit = "SOR", 0.0, 3 if precision == "fp64" else 2
+    g = case.grid
+    rng = np.random.default_rng(11)
+    b, x0 = np.zeros(g.n), np.zeros(g.n)
+    interior(b, g)[...] = rng.standard_normal(interior(b, g).shape).astype(np.float32)
+    interior(x0, g)[...] = 0.1 * rng.standard_normal(interior(b, g).shape).astype(np.float32)
+    outs = []
+    for no_tma in ("0", "1"):
+        monkeypatch.setenv("FALM_B200_NO_TMA", no_tma)
+        ctx = make_ctx(case, precision)
+        xd, bd, rd = dev(ctx, x0), dev(ctx, b), ctx.field(1)
+        ctx.solve(xd, bd, rd)
+        outs.append(interior(host(xd), g).copy())
+    assert np.isfinite(outs[0]).all()
+    assert rel_l2(outs[0], outs[1]) < (5e-11 if precision == "fp64" else 2e-5)
+
+
 def test_pbicgstab_converged(oracle, lib_built):
     case = CASES["cavity"]()
     case.tol = 1e-10
