@@ -431,6 +431,20 @@ int pc_mv_launch(falm_ctx *ctx, cudaStream_t st, const T *r, T *z) {
     return FALM_OK;
 }
 
+// Whether the plane streams' boxes can be copied by the blocks' threads where TMA
+// cannot (BoxCopy): two guide cells on every side, as the boxes' halos assume.
+// Before, such grids ran the row kernels, which recompute the metric of every
+// neighbour and read every neighbour through L1: the pseudo-velocity of the
+// 301 x 157 x 131 channel 387 us in FP32 (180 copied), face velocity + residual
+// 72 + 85 (108), the check 85 (46), SGS 118 (103), projection 83 (69); in FP64 861
+// (242), 126 + 114 (139), SGS 207 (147), projection 157 (119).  A body's kMinCopied:
+// cells below which its row kernel is the faster one, on small grids where a plane
+// stream is bound by the latency of its planes (63^3: SGS 13 us against 20,
+// projection 6 against 12; 101^3: equal within 15% either way).
+bool cpa_ok(const falm_ctx *ctx) { return ctx->geo.gc == 2; }
+template <class Body, class = void> struct P3MinCopied { static constexpr long long v = 0; };
+template <class Body> struct P3MinCopied<Body, std::void_t<decltype(Body::kMinCopied)>> { static constexpr long long v = Body::kMinCopied; };
+
 // ring depth of the multi-field plane stream: keep >= 2 planes in flight and
 // at least two CTAs per SM
 template <typename T, int NF> struct P3Conf { static constexpr int NS = NF > 1 ? 4 : 6; };
@@ -449,24 +463,32 @@ int p3_launch(falm_ctx *ctx, int cls, cudaStream_t st, const Region3 &R, int org
     if (ctx->no_tma) return 0;
     using L = P3Layout<T, NF, P3Rows<T, Body>::v>;
     constexpr int NS = P3NS<T, NF, Body>::v;
-    MapSet<NF> maps;
     int slot = 0;
-    for (int f = 0; f < NF; f++) {
-        if (!make_map(ctx, &maps.m[f], (const T *)ptr[f], ncomp[f], L::BX, L::BY)) return 0;
-        maps.ncomp[f] = ncomp[f];
-        slot += ncomp[f] * L::FB;
-    }
+    for (int f = 0; f < NF; f++) slot += ncomp[f] * L::FB;
     // the kernel lays the slot out from the body's component counts
     if (slot != (Body::NC0 + Body::NC1) * L::FB) return -fail(ctx, FALM_ERR_ARG, "plane stream: field components do not match the body");
     const int smem = NS * slot + 256;
     const int bx = (R.i1 - R.i0 + L::TX - 1) / L::TX, by = (R.j1 - R.j0 + L::TY - 1) / L::TY;
-    auto kern = k_plane3_tma<T, NF, NS, NV, Body>;
-    const int kc = chunk_len(ctx, (long long)bx * by, R.k1 - R.k0, resident_per_sm(kern, 256, smem), 64, 2);
-    dim3 grid(bx, by, (R.k1 - R.k0 + kc - 1) / kc);
-    if ((long long)grid.x * grid.y * grid.z > ctx->red.maxBlocks) return 0;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int rc = launch_k(ctx, cls, st, [&] { kern<<<grid, 256, smem, st>>>(ctx->geo, R, org, kc, maps, body, ctx->red, ctx->kerr); });
-    return rc ? -rc : 1;
+    auto launch = [&](auto kern, const auto &src) -> int {
+        const int kc = chunk_len(ctx, (long long)bx * by, R.k1 - R.k0, resident_per_sm(kern, 256, smem), 64, 2);
+        const dim3 grid(bx, by, (R.k1 - R.k0 + kc - 1) / kc);
+        if ((long long)grid.x * grid.y * grid.z > ctx->red.maxBlocks) return 0;
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const int rc = launch_k(ctx, cls, st, [&] { kern<<<grid, 256, smem, st>>>(ctx->geo, R, org, kc, src, body, ctx->red, ctx->kerr); });
+        return rc ? -rc : 1;
+    };
+    MapSet<NF> maps;
+    bool tma = true;
+    for (int f = 0; f < NF && tma; f++) {
+        tma = make_map(ctx, &maps.m[f], (const T *)ptr[f], ncomp[f], L::BX, L::BY);
+        maps.ncomp[f] = ncomp[f];
+    }
+    if (tma) return launch(k_plane3_tma<T, NF, NS, NV, false, Body>, maps);
+    const Geom &g = ctx->geo;
+    if (!cpa_ok(ctx) || (long long)g.nx * g.ny * g.nz < P3MinCopied<Body>::v) return 0;
+    SrcSet<T, NF> src;
+    for (int f = 0; f < NF; f++) src.p[f] = (const T *)ptr[f];
+    return launch(k_plane3_tma<T, NF, NS, NV, true, Body>, src);
 }
 
 #define P3_OR(CLS, ST, T_, NF_, NV_, R_, ORG_, PTRS_, NCOMP_, BODY_, ROWLAUNCH)            \

@@ -14,6 +14,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "poisson.cuh"
+#include "poisson_tma.cuh"
 #include "tma.cuh"
 
 namespace fb {
@@ -82,8 +83,10 @@ template <typename T, class Body> struct P3Rows<T, Body, std::void_t<decltype(Bo
 //       const ZS&, acc); void finish(tot)
 // The pointwise operands of a plane are loaded before the wait for the plane
 // ahead, for every row of the thread, so their latency overlaps the wait.
-template <typename T, int NF, int NS, int NV, class Body>
-__global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g, Region3 R, int org, int kc, const __grid_constant__ MapSet<NF> maps,
+// CPA: the boxes are copied by the block's threads (SrcSet) instead of by TMA (MapSet).
+template <typename T, int NF, int NS, int NV, bool CPA, class Body>
+__global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g, Region3 R, int org, int kc,
+                                                  const __grid_constant__ std::conditional_t<CPA, SrcSet<T, NF>, MapSet<NF>> maps,
                                                   Body body, RedWork rw, int *err) {
     using L = P3Layout<T, NF, P3Rows<T, Body>::v>;
     extern __shared__ unsigned char smem_raw[];
@@ -103,7 +106,10 @@ __global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g
     P3View<T, NF, L::RY> v;
     v.foff[0] = 0;
     if (NF > 1) v.foff[NF - 1] = FOFF1;
-    const int xb = box_origin(i0 - org, L::BX, g.sx, 16 / (int)sizeof(T)), yb = box_origin(j0 - 1, L::BY, g.sy, 1);
+    const int xb = CPA ? i0 - org : box_origin(i0 - org, L::BX, g.sx, 16 / (int)sizeof(T)), yb = CPA ? j0 - 1 : box_origin(j0 - 1, L::BY, g.sy, 1);
+    BoxCopy<L::BX, L::PE, 256> bc;
+    if constexpr (CPA) bc.init(xb, yb, g.sx, g.sy);
+    const bool lead = CPA || threadIdx.x == 0;   // issues the copies
     const int ox = min(i, R.i1 - 1) - xb;
     int jr[RY], orr[RY];
     bool act[RY];
@@ -142,6 +148,15 @@ __global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g
     auto issue = [&](int q, int s) {
         uint64_t *b = bar + s;
         unsigned char *dst = smem + s * SLOTB;
+        if constexpr (CPA) {
+            const long long c = (long long)(P0 + q) * g.sx * g.sy;
+#pragma unroll
+            for (int f = 0; f < NF; f++)
+#pragma unroll
+                for (int d = 0; d < (f ? Body::NC1 : Body::NC0); d++) bc.copy((T *)(dst + (f ? FOFF1 : 0)) + d * L::PE, maps.p[f] + c + d * g.n);
+            cp_async_arrive(b);
+            return;
+        } else {
         bool ok = true;
 #pragma unroll
         for (int f = 0; f < NF; f++) ok = ok && tma_ok(dst + (f ? FOFF1 : 0), xb, yb, P0 + q, (int)sizeof(T), g.sx, g.sy, g.sz);
@@ -152,19 +167,22 @@ __global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g
         mbar_expect_tx(b, TXB);
 #pragma unroll
         for (int f = 0; f < NF; f++) tma_load_4d(dst + (f ? FOFF1 : 0), &maps.m[f], xb, yb, P0 + q, 0, b);
+        }
     };
     // warp 0 polls the barriers; the block barrier that follows makes the
     // landed planes visible to every thread
     auto wait_s = [&](int s, int parity) -> bool { return threadIdx.x >= 32 || mbar_wait(bar + s, parity, err); };
     if (threadIdx.x == 0) {
+        if constexpr (!CPA) {
 #pragma unroll
-        for (int f = 0; f < NF; f++) prefetch_tmap(&maps.m[f]);
-        for (int s = 0; s < NS; s++) mbar_init(bar + s, 1);
+            for (int f = 0; f < NF; f++) prefetch_tmap(&maps.m[f]);
+        }
+        for (int s = 0; s < NS; s++) mbar_init(bar + s, CPA ? 256 : 1);
         mbar_fence_init();
     }
     __syncthreads();
     int issued = min(NS, nplanes), waited = 0;
-    if (threadIdx.x == 0)
+    if (lead)
         for (int q = 0; q < issued; q++) issue(q, q % NS);
     // every plane is waited for exactly once, before its first read: planes 0
     // and 1 here, plane q+1 at iteration q
@@ -205,7 +223,7 @@ __global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g
                 if (__syncthreads_or(fail)) goto drain;
                 // plane q-2 is no longer needed: refill its slot
                 if (q >= 2 && q - 2 + NS < nplanes) {
-                    if (threadIdx.x == 0) { fence_proxy_async(); issue(q - 2 + NS, (u + NS - 2) % NS); }
+                    if (lead) { if (!CPA) fence_proxy_async(); issue(q - 2 + NS, (u + NS - 2) % NS); }
                     issued = q - 2 + NS + 1;
                 }
                 const typename Body::ZS zst = body.plane_state(k);
@@ -253,6 +271,7 @@ struct UtoUUBody {
     T *uu, *rhs;
     T scale;
     static constexpr int NC0 = 3, NC1 = 0;   // field: the velocity to interpolate
+    static constexpr long long kMinCopied = 1 << 20;
     using PW = NoPW;
     using CS = NoPW;
     using ZS = NoPW;
@@ -305,6 +324,7 @@ struct ProjectBody {
     const T *uua;
     T dt;
     static constexpr int NC0 = 1, NC1 = 0;   // field: the pressure
+    static constexpr long long kMinCopied = 1 << 20;
     static constexpr int kMinBlocks = 3;     // FP32: room for the pointwise operands loaded a plane ahead
     // face velocity (f) and cell velocity (a, interior cells only) before the correction
     struct PW { T f0, f1, f2, a0, a1, a2; };
@@ -419,6 +439,46 @@ struct UtoUUResBody {
     }
 };
 
+// ---------------------------------------------------------------- residual body
+// ResBody (a pass residual, or with CHECK the outer check of the true residual)
+// one cell at a time, for rows whose cells cannot be accessed in aligned pairs.
+// Field: x (1 comp); pointwise: b.
+template <typename T, bool CHECK>
+struct P3ResBody {
+    Geom g;
+    MetricView<T> mv;
+    ResBody<T, CHECK> rb;
+    static constexpr int NC0 = 1, NC1 = 0;
+    static constexpr int kMinBlocks = 3;
+    struct PW { T b; };
+    using CS = typename Op7<T>::Col;
+    using ZS = typename Op7<T>::ZPl;
+    __device__ bool skip() const { return rb.skip(); }
+    __device__ PW pw_load(int, int, int, long long c) const { return PW{rb.b[c]}; }
+    __device__ CS col_state(int i, int j) const { return rb.op.column(i, j); }
+    __device__ ZS plane_state(int k) const { return rb.op.zplane(k); }
+    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 1> &v, const ColMet<T> &, const PW &w, const CS &cs, const ZS &zs,
+                         double (&acc)[ResBody<T, CHECK>::NV]) const {
+        const T ac = rb.op.ac_col(cs, zs);
+        double ax = (double)ac * (double)v.at(0, 0, 0);
+        ax = fma((double)cs.ae, (double)v.at(0, 0, 0, 1, 0), ax);
+        ax = fma((double)cs.aw, (double)v.at(0, 0, 0, -1, 0), ax);
+        ax = fma((double)cs.an, (double)v.at(0, 0, 0, 0, 1), ax);
+        ax = fma((double)cs.as, (double)v.at(0, 0, 0, 0, -1), ax);
+        ax = fma((double)zs.at, (double)v.at(0, 0, 1), ax);
+        ax = fma((double)zs.ab, (double)v.at(0, 0, -1), ax);
+        const double rv = (double)w.b - ax;
+        acc[0] += rv * rv;
+        if constexpr (!CHECK) {
+            const T rt = (T)rv;
+            rb.rr[c] = rt;
+            if (rb.pp) rb.pp[c] = pc_first<T>(rb.pc_type, i, j, k + rb.op.t.koff, rt, ac, rb.pc_omega);
+            acc[1] += (double)rt * (double)rt;
+        }
+    }
+    __device__ void finish(const double (&tot)[ResBody<T, CHECK>::NV]) const { rb.finish(tot); }
+};
+
 // ---------------------------------------------------------------- SGS + divergence body
 // Smagorinsky / CSM (src/dev/FalmCFDDevCall.cu:409-555) and the FP64
 // divergence norm (:557-581 + app/nedo/main.cpp:194-197).  Fields: 0 u (3), 1 uu (3).
@@ -433,6 +493,7 @@ struct SgsDivBody {
     T *div_out;
     double *divsum;
     static constexpr int NC0 = 3, NC1 = 3;   // fields: the cell velocity, the face velocity
+    static constexpr long long kMinCopied = 1 << 20;
     static constexpr int kRows64 = 1;        // FP64: a 63 KB ring (2 CTAs per SM) instead of 126 KB
     using PW = NoPW;
     // filter width (cube root of the volume, as cbrt(hx) cbrt(hy) cbrt(hz)) and

@@ -343,12 +343,17 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
     bool pp_ready = first_res_done;
     auto res_pass = [&](int check) -> int {
         int s7;
+        const void *const fx[1] = {x};
+        const int nc[1] = {1};
         if (check) {
-            s7 = s7_launch<T, 1>(ctx, FALM_K_RES, ist, x, ResBody<T, true>{op, b, nullptr, nullptr, sc, 1});
+            const ResBody<T, true> body{op, b, nullptr, nullptr, sc, 1};
+            s7 = s7_launch<T, 1>(ctx, FALM_K_RES, ist, x, body);
+            if (s7 == 0 && !ctx->A_explicit) s7 = p3_launch<T, 1, 1>(ctx, FALM_K_RES, ist, R, 2, fx, nc, P3ResBody<T, true>{g, mview<T>(ctx), body});
         } else {
             ResBody<T> body{op, b, nullptr, rr, sc, 0};
             body.pp = half ? nullptr : first_target(pp); body.pc_type = pct; body.pc_omega = pcw;
             s7 = s7_launch<T, 2>(ctx, FALM_K_RES, ist, x, body);
+            if (s7 == 0 && !ctx->A_explicit) s7 = p3_launch<T, 1, 2>(ctx, FALM_K_RES, ist, R, 2, fx, nc, P3ResBody<T, false>{g, mview<T>(ctx), body});
         }
         if (s7 < 0) return -s7;
         if (s7 == 0) LAUNCH(FALM_K_RES, ist, (k_res<T><<<grid, kRowThreads, 0, ist>>>(g, R, op, x, b, r, rr, ctx->red, sc, check)));

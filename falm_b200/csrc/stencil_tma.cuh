@@ -13,6 +13,7 @@
 #include "cfd.cuh"
 #include "pair.cuh"
 #include "tma.cuh"
+#include <type_traits>
 
 namespace fb {
 
@@ -64,10 +65,11 @@ struct PUTile {
 // race-free FSPseudoU (src/dev/FalmCFDDevCall.cu:10-301), same expressions as
 // k_pseudo_u; one instantiation per advection scheme ADV (FALM_ADV_*), so the
 // three components' arithmetic is straight-line code
-template <typename T, int NS, int ADV>
+// CPA: the boxes are copied by the block's threads (from u, uu and nut) instead of by TMA.
+struct alignas(64) PUMaps { CUtensorMap u, uu, nut; };
+template <typename T, int NS, int ADV, bool CPA>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Geom g, int kc, MetricView<T> mv,
-    const __grid_constant__ CUtensorMap mu, const __grid_constant__ CUtensorMap muu,
-    const __grid_constant__ CUtensorMap mnut, const T *__restrict__ un, int un_is_u, T *__restrict__ ua,
+    const __grid_constant__ std::conditional_t<CPA, SrcSet<T, 3>, PUMaps> src, const T *__restrict__ un, int un_is_u, T *__restrict__ ua,
     const T *__restrict__ ff, AlmFuse af, T ReI, T dt, int *err) {
     constexpr int adv = ADV;
     using L = PUTile<T, NS>;
@@ -84,7 +86,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
     // along the march from q = 2 (NS need not be a power of two)
     int s0 = 2 % NS, s1 = 3 % NS, s2 = 4 % NS, ph2 = (4 / NS) & 1;
     // box origin (tile minus the halo of 2), kept inside the tensor when it is wide enough
-    const int xb = box_origin(i0 - 2, L::BX, g.sx, 16 / (int)sizeof(T)), yb = box_origin(j0 - 2, L::BY, g.sy, 1);
+    const int xb = CPA ? i0 - 2 : box_origin(i0 - 2, L::BX, g.sx, 16 / (int)sizeof(T)), yb = CPA ? j0 - 2 : box_origin(j0 - 2, L::BY, g.sy, 1);
+    BoxCopy<L::BX, L::PE, 256> bc;
+    if constexpr (CPA) bc.init(xb, yb, g.sx, g.sy);
+    const bool lead = CPA || threadIdx.x == 0;   // issues the copies
     const int ox = min(i, g.sx - g.gc - 1) - xb, oy = min(j, g.sy - g.gc - 1) - yb;
     const int o = oy * L::BX + ox;
     // self-check: the radius-2 neighbourhood of a computed cell lies inside the staged box
@@ -93,15 +98,25 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
     auto issue = [&](int q) {
         unsigned char *s = slot(q);
         uint64_t *b = bar + (q % NS);
+        if constexpr (CPA) {
+            const long long c = (long long)(P0 + q) * g.sx * g.sy;
+#pragma unroll
+            for (int d = 0; d < 7; d++) {
+                const int f = d < 3 ? 0 : (d < 6 ? 1 : 2), m = d - 3 * f;
+                bc.copy((T *)(s + f * L::U_BYTES) + m * L::PE, src.p[f] + c + m * N);
+            }
+            cp_async_arrive(b);
+        } else {
         const int e = (int)sizeof(T);
         if (tma_ok(s, xb, yb, P0 + q, e, g.sx, g.sy, g.sz) && tma_ok(s + L::U_BYTES, xb, yb, P0 + q, e, g.sx, g.sy, g.sz) &&
             tma_ok(s + 2 * L::U_BYTES, xb, yb, P0 + q, e, g.sx, g.sy, g.sz)) {
             mbar_expect_tx(b, L::TX_BYTES);
-            tma_load_4d(s, &mu, xb, yb, P0 + q, 0, b);
-            tma_load_4d(s + L::U_BYTES, &muu, xb, yb, P0 + q, 0, b);
-            tma_load_4d(s + 2 * L::U_BYTES, &mnut, xb, yb, P0 + q, 0, b);
+            tma_load_4d(s, &src.u, xb, yb, P0 + q, 0, b);
+            tma_load_4d(s + L::U_BYTES, &src.uu, xb, yb, P0 + q, 0, b);
+            tma_load_4d(s + 2 * L::U_BYTES, &src.nut, xb, yb, P0 + q, 0, b);
         } else {
             tma_reject(b, err, 1);
+        }
         }
     };
     // column constants (x, y metric factors and the ALM distance in x/y) and the
@@ -132,13 +147,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
     }
     int issued = 0, waited = 0;
     if (threadIdx.x == 0) {
-        prefetch_tmap(&mu); prefetch_tmap(&muu); prefetch_tmap(&mnut);
-        for (int s = 0; s < NS; s++) mbar_init(bar + s, 1);
+        if constexpr (!CPA) { prefetch_tmap(&src.u); prefetch_tmap(&src.uu); prefetch_tmap(&src.nut); }
+        for (int s = 0; s < NS; s++) mbar_init(bar + s, CPA ? 256 : 1);
         mbar_fence_init();
     }
     __syncthreads();
     const int first = min(NS, nplanes);
-    if (threadIdx.x == 0)
+    if (lead)
         for (int q = 0; q < first; q++) issue(q);
     issued = first;
     // warp 0 polls the barriers; the block barrier that follows makes the
@@ -167,8 +182,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
     {
         const int upto = min(NS + 1, nplanes - 1);
         if (upto >= issued) {
-            if (threadIdx.x == 0) {
-                fence_proxy_async();
+            if (lead) {
+                if (!CPA) fence_proxy_async();
                 for (int pl = issued; pl <= upto; pl++) issue(pl);
             }
             issued = upto + 1;
@@ -182,8 +197,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
         {   // planes up to q-1 are no longer read (held in registers): refill their slots
             const int upto = min(q - 1 + NS, nplanes - 1);
             if (upto >= issued) {
-                if (threadIdx.x == 0) {
-                    fence_proxy_async();
+                if (lead) {
+                    if (!CPA) fence_proxy_async();
                     for (int pl = issued; pl <= upto; pl++) issue(pl);
                 }
                 issued = upto + 1;

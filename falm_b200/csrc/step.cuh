@@ -35,44 +35,42 @@ int pseudo_u_t(falm_ctx *ctx, const T *un, const T *u, const T *uu, T *ua, const
     const Geom &g = ctx->geo;
     constexpr int NS = PUConf<T>::NS;
     using L = PUTile<T, NS>;
-    CUtensorMap mu, muu, mnut;
-    if (!ctx->no_tma && make_map(ctx, &mu, u, 3, L::BX, L::BY) && make_map(ctx, &muu, uu, 3, L::BX, L::BY) &&
-        make_map(ctx, &mnut, nut, 1, L::BX, L::BY)) {
-        // FP32 with a 4th-order scheme and an even interior width: the x-pair kernel
-        if constexpr (sizeof(T) == 4) {
-            if (!ctx->pu_v1 && (g.nx & 1) == 0 &&
-                (ctx->adv == FALM_ADV_UPWIND3 || ctx->adv == FALM_ADV_UTOPIA || ctx->adv == FALM_ADV_KK)) {
-                // a ring of 4 planes (49 KB) and at most 128 registers: 4 CTAs per SM
-                constexpr int NS2 = 4;
-                using L = PUTile<T, NS2>;
-                auto k2 = k_pseudo_u_tma2<NS2, FALM_ADV_UPWIND3>;
-                if (ctx->adv == FALM_ADV_UTOPIA) k2 = k_pseudo_u_tma2<NS2, FALM_ADV_UTOPIA>;
-                if (ctx->adv == FALM_ADV_KK) k2 = k_pseudo_u_tma2<NS2, FALM_ADV_KK>;
-                const int bx = (g.nx + L::TX - 1) / L::TX, by = (g.ny + L::TY - 1) / L::TY;
-                const int kc = chunk_len(ctx, (long long)bx * by, g.nz, resident_per_sm(k2, 128, L::SMEM), 64, 4);
-                cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
-                dim3 grid(bx, by, (g.nz + kc - 1) / kc);
-                LAUNCH(FALM_K_PSEUDO_U, st, k2<<<grid, 128, L::SMEM, st>>>(g, kc, mview<T>(ctx), mu, muu, mnut, un, un == u ? 1 : 0, ua, ff, af,
-                                                                         (T)(1.0 / ctx->Re), (T)dt, ctx->kerr));
-                return FALM_OK;
-            }
-        }
-        auto kern = k_pseudo_u_tma<T, NS, FALM_ADV_KK>;
-        switch (ctx->adv) {
-            case FALM_ADV_UPWIND1: kern = k_pseudo_u_tma<T, NS, FALM_ADV_UPWIND1>; break;
-            case FALM_ADV_UPWIND3: kern = k_pseudo_u_tma<T, NS, FALM_ADV_UPWIND3>; break;
-            case FALM_ADV_QUICK: kern = k_pseudo_u_tma<T, NS, FALM_ADV_QUICK>; break;
-            case FALM_ADV_UTOPIA: kern = k_pseudo_u_tma<T, NS, FALM_ADV_UTOPIA>; break;
-            default: break;
-        }
-        const int bx = (g.nx + L::TX - 1) / L::TX, by = (g.ny + L::TY - 1) / L::TY;
-        const int kc = chunk_len(ctx, (long long)bx * by, g.nz, resident_per_sm(kern, 256, L::SMEM), 64, 4);
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
-        dim3 grid(bx, by, (g.nz + kc - 1) / kc);
-        LAUNCH(FALM_K_PSEUDO_U, st, kern<<<grid, 256, L::SMEM, st>>>(g, kc, mview<T>(ctx), mu, muu, mnut, un, un == u ? 1 : 0, ua, ff, af,
-                                                                    (T)(1.0 / ctx->Re), (T)dt, ctx->kerr));
+    PUMaps maps;
+    const bool tma = !ctx->no_tma && make_map(ctx, &maps.u, u, 3, L::BX, L::BY) && make_map(ctx, &maps.uu, uu, 3, L::BX, L::BY) &&
+                     make_map(ctx, &maps.nut, nut, 1, L::BX, L::BY);
+    const int bx = (g.nx + L::TX - 1) / L::TX, by = (g.ny + L::TY - 1) / L::TY;
+    const T ReI = (T)(1.0 / ctx->Re);
+    auto launch = [&](auto kern, int threads, int smem, const auto &...src) -> int {
+        const int kc = chunk_len(ctx, (long long)bx * by, g.nz, resident_per_sm(kern, threads, smem), 64, 4);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const dim3 grid(bx, by, (g.nz + kc - 1) / kc);
+        LAUNCH(FALM_K_PSEUDO_U, st, kern<<<grid, threads, smem, st>>>(g, kc, mview<T>(ctx), src..., un, un == u ? 1 : 0, ua, ff, af, ReI, (T)dt, ctx->kerr));
         return FALM_OK;
+    };
+    if constexpr (sizeof(T) == 4) {
+        // FP32 with a 4th-order scheme and an even interior width: the x-pair kernel, a
+        // ring of 4 planes (49 KB) and at most 128 registers: 4 CTAs per SM
+        if (tma && !ctx->pu_v1 && (g.nx & 1) == 0 && (ctx->adv == FALM_ADV_UPWIND3 || ctx->adv == FALM_ADV_UTOPIA || ctx->adv == FALM_ADV_KK)) {
+            constexpr int NS2 = 4;
+            auto k2 = k_pseudo_u_tma2<NS2, FALM_ADV_UPWIND3>;
+            if (ctx->adv == FALM_ADV_UTOPIA) k2 = k_pseudo_u_tma2<NS2, FALM_ADV_UTOPIA>;
+            if (ctx->adv == FALM_ADV_KK) k2 = k_pseudo_u_tma2<NS2, FALM_ADV_KK>;
+            return launch(k2, 128, PUTile<T, NS2>::SMEM, maps.u, maps.uu, maps.nut);
+        }
     }
+    // one cell per thread, per scheme; the boxes by TMA, or copied by the threads
+    auto pick = [&](auto CPA, const auto &src) -> int {
+        constexpr bool C = decltype(CPA)::value;
+        switch (ctx->adv) {
+            case FALM_ADV_UPWIND1: return launch(k_pseudo_u_tma<T, NS, FALM_ADV_UPWIND1, C>, 256, L::SMEM, src);
+            case FALM_ADV_UPWIND3: return launch(k_pseudo_u_tma<T, NS, FALM_ADV_UPWIND3, C>, 256, L::SMEM, src);
+            case FALM_ADV_QUICK: return launch(k_pseudo_u_tma<T, NS, FALM_ADV_QUICK, C>, 256, L::SMEM, src);
+            case FALM_ADV_UTOPIA: return launch(k_pseudo_u_tma<T, NS, FALM_ADV_UTOPIA, C>, 256, L::SMEM, src);
+            default: return launch(k_pseudo_u_tma<T, NS, FALM_ADV_KK, C>, 256, L::SMEM, src);
+        }
+    };
+    if (tma) return pick(std::false_type{}, maps);
+    if (!ctx->no_tma && cpa_ok(ctx)) return pick(std::true_type{}, SrcSet<T, 3>{{u, uu, nut}});
     LAUNCH(FALM_K_PSEUDO_U, st, k_pseudo_u<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(ctx->geo, R, mview<T>(ctx), un, u, uu, ua, nut, ff, af,
                                                             (T)(1.0 / ctx->Re), (T)dt, ctx->adv));
     return FALM_OK;

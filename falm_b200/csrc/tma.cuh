@@ -107,6 +107,49 @@ __device__ __forceinline__ void tma_reject(uint64_t *bar, int *err, int site) {
     mbar_arrive(bar);
 }
 
+// ---- boxes copied by the block's threads (cp.async), for rows that TMA cannot address
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+// one of the barrier's arrivals once this thread's copies so far have landed (the barrier counts the block's threads)
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// How a plane stream fetches its boxes: by TMA (an elected thread, a tensor map
+// per field), or element by element by all threads of the block with cp.async,
+// for fields whose rows are not a multiple of 16 bytes or whose grid is smaller
+// than a box.  Box elements outside the grid are left out (repeating the last
+// element inside, lanes of one copy on the same address, took 1.7 times as long);
+// no computed cell reads them.
+template <typename T, int NF>
+struct SrcSet {
+    const T *p[NF];
+};
+template <int BX, int PE, int NT>
+struct BoxCopy {
+    static constexpr int E = (PE + NT - 1) / NT;   // box elements of a thread
+    int off[E];                                    // of the plane's element, in elements; -1: outside
+    __device__ __forceinline__ void init(int xb, int yb, int sx, int sy) {
+#pragma unroll
+        for (int n = 0; n < E; n++) {
+            const int e = threadIdx.x + n * NT;
+            const int y = yb + e / BX, x = xb + e % BX;
+            off[n] = e < PE && x < sx && y < sy ? y * sx + x : -1;
+        }
+    }
+    // one component's box of the plane at src
+    template <typename T>
+    __device__ __forceinline__ void copy(T *dst, const T *src) const {
+#pragma unroll
+        for (int n = 0; n < E; n++) {
+            if (off[n] >= 0) cp_async<sizeof(T)>(dst + threadIdx.x + n * NT, src + off[n]);
+        }
+    }
+};
+
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
