@@ -359,6 +359,17 @@ __global__ void __launch_bounds__(256) k_adj_alm_project(Geom g, AlmDev a, const
 #pragma unroll
     for (int s = 0; s < kMaxTurbines; s++)
         if (s == tid) { for (int d = 0; d < 3; d++) { lo[d] = a.bs.lo[s][d]; ex[d] = a.bs.ext[s][d]; } }
+    // the part of the box within the cutoff of the point (the whole box for every point took 194 us at 128 x 64 x 64)
+    {
+        const double rc = sqrt(a.rcut2), p[3] = {px, py, pz};
+        const double *const tab[3] = {xc, yc, zc};
+        const int dim[3] = {g.sx, g.sy, g.sz};
+        for (int d = 0; d < 3; d++) {
+            const int l = max(lo[d], find_index(tab[d], p[d] - rc, dim[d])), h = min(lo[d] + ex[d], find_index(tab[d], p[d] + rc, dim[d]) + 1);
+            lo[d] = l;
+            ex[d] = max(h - l, 0);
+        }
+    }
     double acc[3] = {0, 0, 0};
     const long long tot = (long long)ex[0] * ex[1] * ex[2];
     for (long long q = threadIdx.x; q < tot; q += blockDim.x) {

@@ -146,20 +146,31 @@ __global__ void __launch_bounds__(256) k_alm_force(Geom g, AlmDev a, const doubl
         if (keep) { s_tq[ap] = fabs(ft) * apr; s_th[ap] = fx; }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const double *pxyz = keep ? s_xyz : a.ap_xyz, *ptq = keep ? s_tq : a.ap_torque, *pth = keep ? s_th : a.ap_thrust;
-        double bb[6] = {1e300, -1e300, 1e300, -1e300, 1e300, -1e300};
-        for (int ap = 0; ap < a.apcount; ap++)
-            for (int d = 0; d < 3; d++) {
-                bb[2 * d] = fmin(bb[2 * d], pxyz[3 * ap + d]);
-                bb[2 * d + 1] = fmax(bb[2 * d + 1], pxyz[3 * ap + d]);
+    // the bounding box, one bound per warp, and the turbines' sums, each added in
+    // the points' order by one thread (all of it on one thread took 9 of the
+    // kernel's 22 us at 96 points)
+    {
+        const double *pxyz = keep ? s_xyz : a.ap_xyz;
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (w < 6) {
+            const bool hi = w & 1;
+            double v = hi ? -1e300 : 1e300;
+            for (int ap = lane; ap < a.apcount; ap += 32) {
+                const double x = pxyz[3 * ap + (w >> 1)];
+                v = hi ? fmax(v, x) : fmin(v, x);
             }
-        for (int q = 0; q < 6; q++) a.scal->bbox[q] = bb[q];
-        for (int tid = 0; tid < a.n_turbine && tid < kMaxTurbines; tid++) {
-            double tq = 0, th = 0;
-            for (int q = 0; q < nappt; q++) { tq += ptq[tid * nappt + q]; th += pth[tid * nappt + q]; }
-            a.scal->torque[tid] = tq;
-            a.scal->thrust[tid] = th;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double x = __shfl_xor_sync(0xffffffffu, v, o);
+                v = hi ? fmax(v, x) : fmin(v, x);
+            }
+            if (lane == 0) a.scal->bbox[w] = v;
+        } else if (lane < a.n_turbine && lane < kMaxTurbines) {
+            const double *p = (w == 6 ? (keep ? s_tq : a.ap_torque) : (keep ? s_th : a.ap_thrust)) + lane * nappt;
+            double sum = 0;
+#pragma unroll 8
+            for (int q = 0; q < nappt; q++) sum += p[q];
+            (w == 6 ? a.scal->torque : a.scal->thrust)[lane] = sum;
         }
     }
 }
@@ -187,40 +198,77 @@ __device__ __forceinline__ T cut_bound(double r2) {
     else return r2;
 }
 
-// the APs' positions and forces, converted to T once per block
+// The actuator points in shared memory, converted to T once per block, with the
+// bounding boxes of groups of kApGroup consecutive points (a stretch of a blade):
+// a cell visits the points of the groups within the cutoff of it, about two
+// of twelve in the rotor's box, in the points' order.
+constexpr int kApGroup = 8;
 template <typename T>
-__device__ __forceinline__ void stage_aps(const AlmDev &a, T *s_ap) {
+struct ApStage {
+    T ap[6 * kMaxFusedAp];                                     // position, force
+    T box[6 * ((kMaxFusedAp + kApGroup - 1) / kApGroup)];      // lower and upper bound per axis
+};
+template <typename T>
+__device__ __forceinline__ void stage_aps(const AlmDev &a, ApStage<T> &s) {
     for (int q = threadIdx.x; q < a.apcount; q += blockDim.x) {
-        for (int d = 0; d < 3; d++) { s_ap[6 * q + d] = (T)a.ap_xyz[3 * q + d]; s_ap[6 * q + 3 + d] = (T)a.ap_force[3 * q + d]; }
+        for (int d = 0; d < 3; d++) { s.ap[6 * q + d] = (T)a.ap_xyz[3 * q + d]; s.ap[6 * q + 3 + d] = (T)a.ap_force[3 * q + d]; }
     }
-}
-
-// DistributeAPForce (src/alm/almDevCall.cu:255-294) as a stored field, truncated at rcut
-template <typename T>
-__global__ void __launch_bounds__(kRowThreads) k_alm_project(Geom g, Region3 R, MetricView<T> mv, AlmDev a, T *__restrict__ ff) {
-    __shared__ T s_ap[6 * kMaxFusedAp];
-    const int na = a.apcount;
-    stage_aps<T>(a, s_ap);
     __syncthreads();
-    const T rcut2 = cut_bound<T>(a.rcut2);
-    const double eps = a.euler_eps, sq = sqrt(3.14159265358979323846) * eps, eta = 1. / (sq * sq * sq);
-    const long long N = g.n;
-    FB_FOR_ROWS(R, j, k) FB_FOR_I(R, i) {
-        long long c = g.id(i, j, k);
-        T cx = ldg(mv.m.x[0] + i), cy = ldg(mv.m.x[1] + j), cz = ldg(mv.m.x[2] + k);
-        T fx = 0, fy = 0, fz = 0;
-        const T te = (T)eta, e2 = (T)eps * (T)eps;
-        for (int q = 0; q < na; q++) {
-            T dx = cx - s_ap[6 * q], dy = cy - s_ap[6 * q + 1], dz = cz - s_ap[6 * q + 2];
+    const int ng = (a.apcount + kApGroup - 1) / kApGroup;
+    for (int q = threadIdx.x; q < 3 * ng; q += blockDim.x) {
+        const int gq = q / 3, d = q % 3, e = min((gq + 1) * kApGroup, a.apcount);
+        T lo = s.ap[6 * gq * kApGroup + d], hi = lo;
+        for (int p = gq * kApGroup + 1; p < e; p++) { lo = min(lo, s.ap[6 * p + d]); hi = max(hi, s.ap[6 * p + d]); }
+        s.box[6 * gq + d] = lo;
+        s.box[6 * gq + 3 + d] = hi;
+    }
+    __syncthreads();
+}
+// sum of the points' Gaussians at a cell, truncated at the cutoff (DistributeAPForce, src/alm/almDevCall.cu:255-294)
+template <typename T>
+__device__ __forceinline__ void ap_sum(const ApStage<T> &s, int na, T cx, T cy, T cz, T rcut2, T te, T e2, T &fx, T &fy, T &fz) {
+    const T near2 = rcut2 * T(1.0001);   // a group's box may round to either side of the cutoff
+    for (int g0 = 0, gq = 0; g0 < na; g0 += kApGroup, gq++) {
+        const T *b = s.box + 6 * gq;
+        const T bx = max(max(b[0] - cx, cx - b[3]), T(0)), by = max(max(b[1] - cy, cy - b[4]), T(0)), bz = max(max(b[2] - cz, cz - b[5]), T(0));
+        if (bx * bx + by * by + bz * bz > near2) continue;
+        const int e = min(g0 + kApGroup, na);
+        for (int p = g0; p < e; p++) {
+            const T *q = s.ap + 6 * p;
+            T dx = cx - q[0], dy = cy - q[1], dz = cz - q[2];
             T rr2 = dx * dx + dy * dy + dz * dz;
             if (rr2 < rcut2) {
                 T ex = exp(-rr2 / e2);
-                fx += s_ap[6 * q + 3] * te * ex;
-                fy += s_ap[6 * q + 4] * te * ex;
-                fz += s_ap[6 * q + 5] * te * ex;
+                fx += q[3] * te * ex;
+                fy += q[4] * te * ex;
+                fz += q[5] * te * ex;
             }
         }
-        ff[c] = fx; ff[c + N] = fy; ff[c + 2 * N] = fz;
+    }
+}
+
+// DistributeAPForce (src/alm/almDevCall.cu:255-294) as a stored field, truncated at
+// rcut; a cell farther than that from the points' bounding box is zero at once
+// (every cell against every point: 131 us on the 192 x 96 x 90 channel in FP64)
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads) k_alm_project(Geom g, Region3 R, MetricView<T> mv, MetricView<double> m64, AlmDev a, T *__restrict__ ff) {
+    __shared__ ApStage<T> s_ap;
+    stage_aps<T>(a, s_ap);
+    const T rcut2 = cut_bound<T>(a.rcut2);
+    const double eps = a.euler_eps, sq = sqrt(3.14159265358979323846) * eps, eta = 1. / (sq * sq * sq);
+    const T te = (T)eta, e2 = (T)eps * (T)eps;
+    const double *bb = a.scal->bbox;
+    const double b0 = bb[0], b1 = bb[1], b2 = bb[2], b3 = bb[3], b4 = bb[4], b5 = bb[5];
+    const long long N = g.n;
+    FB_FOR_ROWS(R, j, k) {
+        const double dyz = box_dist2(ldg(m64.m.x[1] + j), b2, b3) + box_dist2(ldg(m64.m.x[2] + k), b4, b5);
+        FB_FOR_I(R, i) {
+            long long c = g.id(i, j, k);
+            T fx = 0, fy = 0, fz = 0;
+            if (box_dist2(ldg(m64.m.x[0] + i), b0, b1) + dyz < a.rcut2)
+                ap_sum<T>(s_ap, a.apcount, ldg(mv.m.x[0] + i), ldg(mv.m.x[1] + j), ldg(mv.m.x[2] + k), rcut2, te, e2, fx, fy, fz);
+            ff[c] = fx; ff[c + N] = fy; ff[c + 2 * N] = fz;
+        }
     }
 }
 
@@ -228,10 +276,9 @@ __global__ void __launch_bounds__(kRowThreads) k_alm_project(Geom g, Region3 R, 
 // farther than the cutoff from the AP bounding box get zero without the AP loop.
 template <typename T>
 __global__ void __launch_bounds__(256) k_alm_box(AlmDev a, const double *xc, const double *yc, const double *zc) {
-    __shared__ T s_ap[6 * kMaxFusedAp];
+    __shared__ ApStage<T> s_ap;
     const int na = a.apcount;
     stage_aps<T>(a, s_ap);
-    __syncthreads();
     const T rcut2 = cut_bound<T>(a.rcut2);
     const double eps = a.euler_eps, sq = sqrt(3.14159265358979323846) * eps, eta = 1. / (sq * sq * sq);
     const double *bb = a.scal->bbox;
@@ -254,18 +301,7 @@ __global__ void __launch_bounds__(256) k_alm_box(AlmDev a, const double *xc, con
         const double cxd = xc[i], cyd = yc[j], czd = zc[k];
         T fx = 0, fy = 0, fz = 0;
         if (box_dist2(cxd, b0, b1) + box_dist2(cyd, b2, b3) + box_dist2(czd, b4, b5) < a.rcut2) {
-            const T cx = (T)cxd, cy = (T)cyd, cz = (T)czd;
-            const T te = (T)eta, e2 = (T)eps * (T)eps;
-            for (int p = 0; p < na; p++) {
-                T dx = cx - s_ap[6 * p], dy = cy - s_ap[6 * p + 1], dz = cz - s_ap[6 * p + 2];
-                T rr2 = dx * dx + dy * dy + dz * dz;
-                if (rr2 < rcut2) {
-                    T ex = exp(-rr2 / e2);
-                    fx += s_ap[6 * p + 3] * te * ex;
-                    fy += s_ap[6 * p + 4] * te * ex;
-                    fz += s_ap[6 * p + 5] * te * ex;
-                }
-            }
+            ap_sum<T>(s_ap, na, (T)cxd, (T)cyd, (T)czd, rcut2, (T)eta, (T)eps * (T)eps, fx, fy, fz);
         }
         f[q] = fx; f[q + tot] = fy; f[q + 2 * tot] = fz;
     }

@@ -442,7 +442,7 @@ int slab_step_t(falm_ctx *ctx, const falm_fields *f, double dt, double t, cudaSt
         if ((rc = slab_alm_t<T>(ctx, u, t, st))) return rc;
         if (ff) {
             const Region3 R = interior(g);
-            LAUNCH(FALM_K_ALM, st, k_alm_project<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(g, R, mview<T>(ctx), ctx->alm, ff));
+            LAUNCH(FALM_K_ALM, st, k_alm_project<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(g, R, mview<T>(ctx), mview<double>(ctx), ctx->alm, ff));
         }
     } else if (ctx->rmcp_on) {
         ff = (T *)ctx->w_ff;

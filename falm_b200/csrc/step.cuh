@@ -86,7 +86,7 @@ int alm_run_t(falm_ctx *ctx, const T *u, T *ff, double t, cudaStream_t st, const
                                                                             t_dev));
     if (ff) {
         const Region3 R = interior(ctx->geo);
-        LAUNCH(FALM_K_ALM, st, k_alm_project<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(ctx->geo, R, mview<T>(ctx), ctx->alm, ff));
+        LAUNCH(FALM_K_ALM, st, k_alm_project<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(ctx->geo, R, mview<T>(ctx), mview<double>(ctx), ctx->alm, ff));
     } else if (ctx->alm.bs.total > 0) {
         // force boxes for the fused projection of the plane-streaming pseudo-velocity kernel
         const long long blocks = std::min<long long>((ctx->alm.bs.total + 255) / 256, (long long)ctx->sm_count * 8);

@@ -476,6 +476,24 @@ def test_alm_forces_and_projection(oracle, lib_built):
         assert rel_l2(interior(host(ff_d), g, 3), interior(ff_o, g, 3)) < 1e-13
 
 
+@pytest.mark.parametrize("n_ap", [1, 3, 8, 11, 128])
+def test_alm_projection_of_any_point_count(oracle, lib_built, n_ap):
+    """Groups of eight points cut short (3, 9, 33 points), whole (24) and as many
+    as the kernel holds (384): forces and projection against the oracle."""
+    case = cases.small_channel(40, 28, 28, intensity=0.0, n_ap_per_blade=n_ap)
+    cs, m = _setup(oracle, case)
+    g = case.grid
+    st = random_state(case, seed=22, amp=0.05)
+    ff_o = np.zeros(3 * g.n)
+    out = oracle.alm(cs, st["u"], ff_o, 0.3)
+    ctx = make_ctx(case)
+    ff_d = ctx.field(3)
+    tq, th = ctx.alm_run(dev(ctx, st["u"]), ff_d, 0.3)
+    np.testing.assert_allclose(tq, out["torque"], rtol=1e-12)
+    np.testing.assert_allclose(th, out["thrust"], rtol=1e-12)
+    assert rel_l2(interior(host(ff_d), g, 3), interior(ff_o, g, 3)) < 1e-13
+
+
 def test_alm_pitch_motion(oracle, lib_built):
     """platform pitch motion (src/alm/almDevCall.cu:43-61, src/falmath.h:412-460)"""
     case = cases.small_channel(40, 28, 28, intensity=0.0)
