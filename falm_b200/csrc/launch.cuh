@@ -121,13 +121,14 @@ int resident_per_sm(K kernel, int threads, int smem) {
 }
 
 // z planes per CTA of a plane-streaming kernel: the chunk length kc in
-// [8, cap] that minimises the modelled time ceil(CTAs / resident slots) *
+// [3, cap] that minimises the modelled time ceil(CTAs / resident slots) *
 // (kc + halo + 2): the CTAs run in waves of SMs x per_sm, and a CTA's time
 // grows with its planes (the halo planes included) plus a start-up of about
-// two planes.  Ties keep the longer chunk.
+// two planes.  Ties keep the longer chunk.  (At least 8 planes left grids of less
+// than a wave of tiles, 64 x 64 x 64, with fewer CTAs than SMs.)
 int chunk_len(const falm_ctx *ctx, long long blocks_xy, int nz, int per_sm, int cap, int halo) {
     const long long slots = (long long)ctx->sm_count * std::max(1, per_sm);
-    const int lo = std::min(8, nz), hi = std::max(lo, std::min(cap, nz));
+    const int lo = std::min(3, nz), hi = std::max(lo, std::min(cap, nz));
     int best = hi;
     long long best_t = -1;
     for (int kc = hi; kc >= lo; kc--) {
