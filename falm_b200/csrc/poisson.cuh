@@ -435,11 +435,21 @@ __global__ void __launch_bounds__(kRowThreads) k_mv_dot2(Geom g, Region3 R, Op7<
 
 // x += alpha pp + omega ss; r = s - omega t; ||r||, the next rho.  s and t of an
 // odd iteration may lie in other vectors than an even one's (PCVec).  W: cells
-// per access, 2 where rows and bases allow pairs.
+// per access, 2 where rows and bases allow pairs.  loop: the condition of a
+// recorded loop of iterations, set from the done flag by the last one's kernel
+// (a kernel of its own for that cost 2 us an iteration).
+struct LoopCond {
+    cudaGraphConditionalHandle h;
+    int set;
+};
 template <typename T, int W>
 __global__ void __launch_bounds__(kRowThreads) k_bicg_xr(Geom g, Region3 R, T *x, const T *pp, const T *ss, T *r, const T *s0, const T *t0,
-                                                         const T *s1, const T *t1, const T *rr, RedWork rw, SolverScalars *sc) {
-    if (sc->done) return;
+                                                         const T *s1, const T *t1, const T *rr, RedWork rw, SolverScalars *sc,
+                                                         LoopCond loop) {
+    if (sc->done) {
+        if (loop.set && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop.h, 0u);
+        return;
+    }
     const bool odd = sc->it & 1;
     const T *s = odd ? s1 : s0, *t = odd ? t1 : t0;
     const T alpha = (T)sc->alpha, omega = (T)sc->omega;
@@ -483,6 +493,7 @@ __global__ void __launch_bounds__(kRowThreads) k_bicg_xr(Geom g, Region3 R, T *x
     if (grid_sum<2>(acc, rw, tot) && threadIdx.x == 0) {
         if (sc->defer) { sc->red[0] = tot[0]; sc->red[1] = tot[1]; }
         else derive_xr(sc, tot);
+        if (loop.set) cudaGraphSetConditional(loop.h, sc->done ? 0u : 1u);
     }
 }
 

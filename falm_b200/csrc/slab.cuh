@@ -378,7 +378,7 @@ int slab_solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it
             S7_OR(FALM_K_MV_DOT2, st, T, 2, ss, (MvDot2Body<T>{op, t, s, sc}),
                   (k_mv_dot2<T><<<grid, kRowThreads, 0, st>>>(g, R, op, ss, t, s, ctx->red, sc)));
             if ((rc = slab_derive(ctx, 2, 3, st))) return rc;
-            LAUNCH(FALM_K_BICG_XR, st, (k_bicg_xr<T, 1><<<grid, kRowThreads, 0, st>>>(g, R, x, pp, ss, r, s, t, s, t, rr, ctx->red, sc)));
+            LAUNCH(FALM_K_BICG_XR, st, (k_bicg_xr<T, 1><<<grid, kRowThreads, 0, st>>>(g, R, x, pp, ss, r, s, t, s, t, rr, ctx->red, sc, LoopCond{})));
             if ((rc = slab_derive(ctx, 2, 4, st))) return rc;
             if (++queued < batch) continue;
             CK(cudaMemcpyAsync(ctx->scal_host, sc, sizeof(SolverScalars), cudaMemcpyDeviceToHost, st));

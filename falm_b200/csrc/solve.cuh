@@ -88,10 +88,6 @@ bool use_graph(const falm_ctx *ctx) {
     return !(ctx->profiling || ctx->check_sync || ctx->graph_mode == 0);
 }
 
-__global__ void k_graph_continue(const SolverScalars *sc, cudaGraphConditionalHandle h) {
-    cudaGraphSetConditional(h, sc->done ? 0u : 1u);
-}
-
 // drop every recorded loop and step (the settings they were recorded with changed)
 void graphs_clear(falm_ctx *ctx) {
     if (ctx->graphs) {
@@ -120,7 +116,7 @@ __global__ void k_solver_init(SolverScalars *sc, double gsize, double tol, int m
     z.maxit = maxit;
     *sc = z;
 }
-// a pass has ended: its iterations into the totals
+// a pass has ended with no check behind it: its iterations into the totals
 __global__ void k_pass_end(SolverScalars *sc) {
     sc->it_total += sc->it;
     sc->passes += 1;
@@ -130,10 +126,13 @@ __global__ void k_pass_reset(SolverScalars *sc, int maxit) {
     sc->it = 0;
     sc->maxit = maxit;
 }
-// after the FP64 check of a mixed pass: another pass while the true residual
-// misses the tolerance and passes remain (a breakdown's status is cleared: the
-// pass restarts from the true residual); non-finite data ends the solve (done)
+// after the FP64 check of a mixed pass: its iterations into the totals, and another
+// pass while the true residual misses the tolerance and passes remain (a breakdown's
+// status is cleared: the pass restarts from the true residual); non-finite data ends
+// the solve (done)
 __global__ void k_outer_cond(SolverScalars *sc, cudaGraphConditionalHandle h, int max_passes) {
+    sc->it_total += sc->it;
+    sc->passes += 1;
     const bool more = !sc->done && sc->passes < max_passes;
     if (more) sc->status = FALM_OK;
     cudaGraphSetConditional(h, more ? 1u : 0u);
@@ -190,7 +189,7 @@ struct SolveRec {
 // kernels on `ist`, which points at the capture stream meanwhile); prefix and
 // per_iter: kernel launches of iterations 0-1 and of one later iteration
 int solve_graph(falm_ctx *ctx, const void *x, const void *b, const void *r, int esize, int pp_ready,
-                const std::function<int(int)> &emit, cudaStream_t &ist, cudaGraphExec_t *out, int *prefix, int *per_iter) {
+                const std::function<int(int, LoopCond)> &emit, cudaStream_t &ist, cudaGraphExec_t *out, int *prefix, int *per_iter) {
     for (auto &e : *ctx->graphs)
         if (e.x == x && e.b == b && e.r == r && e.w0 == ctx->w_rr && e.A == ctx->A_explicit && e.esize == esize && e.pp_ready == pp_ready) {
             *out = e.exec; *prefix = e.prefix; *per_iter = e.per_iter;
@@ -203,49 +202,25 @@ int solve_graph(falm_ctx *ctx, const void *x, const void *b, const void *r, int 
     cudaGraphExec_t ex = nullptr;
     const cudaStream_t saved = ist;
     ist = ctx->cap_stream;
-    // capture iterations first..last and the condition kernel into `into`
-    auto capture = [&](cudaGraph_t into, int first, int last, int *count) -> int {
-        if (cudaStreamBeginCaptureToGraph(ist, into, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
-            return fail(ctx, FALM_ERR_CUDA, "solve graph: capture");
+    // iterations first..last into `into` after deps, the last one's kernel setting the loop condition
+    auto capture = [&](cudaGraph_t into, std::vector<cudaGraphNode_t> &deps, int first, int last, int *count) -> int {
         const long long l0 = ctx->launches;
-        int crc = FALM_OK;
-        for (int itp = first; itp <= last && !crc; itp++) crc = emit(itp);
-        if (!crc) {
-            k_graph_continue<<<1, 1, 0, ist>>>(ctx->scal, h);
-            if (cudaGetLastError() != cudaSuccess) crc = fail(ctx, FALM_ERR_CUDA, "solve graph: condition kernel");
-        }
+        const int crc = capture_into(ctx, into, deps, [&]() -> int {
+            int e = FALM_OK;
+            for (int itp = first; itp <= last && !e; itp++) e = emit(itp, LoopCond{h, itp == last ? 1 : 0});
+            return e;
+        });
         *count = (int)(ctx->launches - l0);
         ctx->launches = l0;
-        cudaGraph_t got = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(ist, &got);
-        if (!crc && (e != cudaSuccess || got != into)) crc = fail(ctx, FALM_ERR_CUDA, "solve graph: end of capture");
-        cudaGetLastError();
         return crc;
     };
     int rc = FALM_OK, np = 0, nb = 0;
+    std::vector<cudaGraphNode_t> deps, body_deps;
+    cudaGraph_t body = nullptr;
     if (cudaGraphConditionalHandleCreate(&h, gr, 1, cudaGraphCondAssignDefault) != cudaSuccess) rc = fail(ctx, FALM_ERR_CUDA, "solve graph: handle");
-    if (!rc) rc = capture(gr, 0, 1, &np);
-    if (!rc) {
-        // the loop follows the prefix's last node(s)
-        size_t nn = 0, ne = 0;
-        cudaGraphGetNodes(gr, nullptr, &nn);
-        std::vector<cudaGraphNode_t> nodes(nn);
-        if (nn) cudaGraphGetNodes(gr, nodes.data(), &nn);
-        cudaGraphGetEdges(gr, nullptr, nullptr, &ne);
-        std::vector<cudaGraphNode_t> from(ne), to(ne);
-        if (ne) cudaGraphGetEdges(gr, from.data(), to.data(), &ne);
-        std::vector<cudaGraphNode_t> leaves;
-        for (auto nd : nodes)
-            if (std::find(from.begin(), from.end(), nd) == from.end()) leaves.push_back(nd);
-        cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};   // every other byte zero
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cn;
-        if (cudaGraphAddNode(&cn, gr, leaves.data(), leaves.size(), &cp) != cudaSuccess) rc = fail(ctx, FALM_ERR_CUDA, "solve graph: loop node");
-        else rc = capture(cp.conditional.phGraph_out[0], 2, 2, &nb);
-    }
+    if (!rc) rc = capture(gr, deps, 0, 1, &np);
+    if (!rc) rc = add_while(ctx, gr, deps, h, &body);   // the loop follows the prefix's last node
+    if (!rc) rc = capture(body, body_deps, 2, 2, &nb);
     if (!rc && cudaGraphInstantiate(&ex, gr, 0) != cudaSuccess) rc = fail(ctx, FALM_ERR_CUDA, "solve graph: instantiate");
     ist = saved;
     cudaGetLastError();
@@ -368,16 +343,16 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         return FALM_OK;
     };
     // the x and r update, s and t in s0, t0 at even iterations and in s1, t1 at odd ones
-    auto bicg_xr = [&](const T *s0, const T *t0, const T *s1, const T *t1) -> int {
+    auto bicg_xr = [&](const T *s0, const T *t0, const T *s1, const T *t1, LoopCond loop) -> int {
         const auto k2 = k_bicg_xr<T, 2>, k1 = k_bicg_xr<T, 1>;
         const auto kern = pairs_ok(ctx, x, r) ? k2 : k1;
-        LAUNCH(FALM_K_BICG_XR, ist, kern<<<row_grid_wave(ctx, R, kern), kRowThreads, 0, ist>>>(g, R, x, pp, ss, r, s0, t0, s1, t1, rr, ctx->red, sc));
+        LAUNCH(FALM_K_BICG_XR, ist, kern<<<row_grid_wave(ctx, R, kern), kRowThreads, 0, ist>>>(g, R, x, pp, ss, r, s0, t0, s1, t1, rr, ctx->red, sc, loop));
         return FALM_OK;
     };
     // the kernels of iteration itp of the pass (2 stands for every later
     // one): r equals rr until the first k_bicg_xr, and the first
     // iteration's p equals r, so it reads rr in their place
-    auto emit_iter = [&](int itp) -> int {
+    auto emit_iter = [&](int itp, LoopCond loop) -> int {
         const T *rin = itp == 0 ? rr : r;
         T *pout = itp == 0 ? nullptr : p;
         const T *pin = itp == 1 ? rr : p, *pv = itp == 0 ? rr : p;
@@ -385,7 +360,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         if (half) {   // the vectors of an iteration follow its parity on the device (PCVec)
             if ((erc = pc_mv_launch<T, 0>(ctx, ist, r, pp))) return erc;
             if ((erc = pc_mv_launch<T, 1>(ctx, ist, r, ss))) return erc;
-            if ((erc = bicg_xr(s, t, p, q))) return erc;
+            if ((erc = bicg_xr(s, t, p, q, loop))) return erc;
             return FALM_OK;
         }
         if (!(itp == 0 && pp_ready))
@@ -397,7 +372,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         if ((erc = precondition_rest(ss, s))) return erc;
         S7_OR(FALM_K_MV_DOT2, ist, T, 2, ss, (MvDot2Body<T>{op, t, s, sc}),
               (k_mv_dot2<T><<<grid, kRowThreads, 0, ist>>>(g, R, op, ss, t, s, ctx->red, sc)));
-        if ((erc = bicg_xr(s, t, s, t))) return erc;
+        if ((erc = bicg_xr(s, t, s, t, loop))) return erc;
         return FALM_OK;
     };
     if (rec) {
@@ -416,31 +391,23 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
             ctx->launches = l0;
             return crc;
         };
-        auto cond = [&](cudaGraphConditionalHandle h) -> int {
-            k_graph_continue<<<1, 1, 0, ist>>>(sc, h);
-            return cudaGetLastError() == cudaSuccess ? FALM_OK : fail(ctx, FALM_ERR_CUDA, "graph: condition kernel");
-        };
+        const bool checked_pass = mixed && max_outer > 1;   // k_outer_cond adds up a pass's iterations
         auto rec_pass = [&](cudaGraph_t gr, std::vector<cudaGraphNode_t> &deps) -> int {
             cudaGraphConditionalHandle h;
             if (cudaGraphConditionalHandleCreate(&h, gr, 1, cudaGraphCondAssignDefault) != cudaSuccess)
                 return fail(ctx, FALM_ERR_CUDA, "graph: handle");
             int e = cap(gr, deps, &fixed, [&]() -> int {
-                int q2 = emit_iter(0);
-                if (!q2) q2 = emit_iter(1);
-                if (!q2) q2 = cond(h);
+                int q2 = emit_iter(0, LoopCond{});
+                if (!q2) q2 = emit_iter(1, LoopCond{h, 1});
                 return q2;
             });
             cudaGraph_t body = nullptr;
             if (!e) e = add_while(ctx, gr, deps, h, &body);
             std::vector<cudaGraphNode_t> bd;
             long long pi = 0;
-            if (!e) e = cap(body, bd, &pi, [&]() -> int {
-                int q2 = emit_iter(2);
-                if (!q2) q2 = cond(h);
-                return q2;
-            });
+            if (!e) e = cap(body, bd, &pi, [&]() -> int { return emit_iter(2, LoopCond{h, 1}); });
             per_iter = pi;
-            if (!e) e = cap(gr, deps, &fixed, [&]() -> int {
+            if (!e && !checked_pass) e = cap(gr, deps, &fixed, [&]() -> int {
                 LAUNCH(FALM_K_OTHER, ist, k_pass_end<<<1, 1, 0, ist>>>(sc));
                 return FALM_OK;
             });
@@ -453,7 +420,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
                 return res_pass(0);
             });
         if (!e) e = rec_pass(rec->graph, rec->deps);
-        if (!e && mixed && max_outer > 1) {
+        if (!e && checked_pass) {
             cudaGraphConditionalHandle ho;
             if (cudaGraphConditionalHandleCreate(&ho, rec->graph, 0, cudaGraphCondAssignDefault) != cudaSuccess)
                 e = fail(ctx, FALM_ERR_CUDA, "graph: handle");
@@ -525,7 +492,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
         // queued after convergence returns at once
         int batch = 1, queued = 0;
         for (int itp = 0; !graph; itp++) {
-            if ((rc = emit_iter(itp))) return rc;
+            if ((rc = emit_iter(itp, LoopCond{}))) return rc;
             if (++queued < batch) continue;
             if (want_check && !explicit_check) {
                 ResBody<T, true> cb{op, b, nullptr, nullptr, sc, 1};
