@@ -307,6 +307,42 @@ __global__ void __launch_bounds__(256) k_alm_box(AlmDev a, const double *xc, con
     }
 }
 
+// ua += dt ff at the cells of the force boxes (a cell in several boxes takes the
+// first one's force, which is the sum over all points), or of a stored force field,
+// which is zero outside them.  The step adds the force
+// after the pseudo-velocity, so that the points' evaluation and projection, a
+// chain of two kernels of about 20 us that leave most of the GPU idle, run beside
+// it (RN once more in the box: 2^-53 or 2^-24 of ua).
+template <typename T>
+__global__ void __launch_bounds__(256) k_alm_add(Geom g, AlmDev a, T *ua, const T *ff, T dt) {
+    const int tot = (int)a.bs.total;
+    const T *f = (const T *)a.fbox;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) {
+        int box = 0, l0 = 0, l1 = 0, l2 = 0, e0 = 1, e1 = 1, o = 0;
+#pragma unroll
+        for (int s = 0; s < kMaxTurbines; s++)
+            if (s < a.bs.n && q >= a.bs.off[s]) {
+                box = s;
+                l0 = a.bs.lo[s][0]; l1 = a.bs.lo[s][1]; l2 = a.bs.lo[s][2];
+                e0 = a.bs.ext[s][0]; e1 = a.bs.ext[s][1]; o = (int)a.bs.off[s];
+            }
+        int r = q - o;
+        const int i = l0 + r % e0;
+        r /= e0;
+        const int j = l1 + r % e1, k = l2 + r / e1;
+        bool earlier = false;
+#pragma unroll
+        for (int s = 0; s < kMaxTurbines; s++)
+            if (s < box && (unsigned)(i - a.bs.lo[s][0]) < (unsigned)a.bs.ext[s][0] && (unsigned)(j - a.bs.lo[s][1]) < (unsigned)a.bs.ext[s][1] &&
+                (unsigned)(k - a.bs.lo[s][2]) < (unsigned)a.bs.ext[s][2])
+                earlier = true;
+        if (earlier) continue;
+        const long long c = g.id(i, j, k);
+#pragma unroll
+        for (int d = 0; d < 3; d++) ua[c + d * g.n] += dt * (ff ? ff[c + d * g.n] : f[q + d * tot]);
+    }
+}
+
 // ---------------------------------------------------------------- boundary conditions
 // previous-velocity view for the convective outlet: full field or the
 // compact 3-plane copy [d][plane][k][j], planes i = sx-gc-2, sx-gc-1, sx-gc

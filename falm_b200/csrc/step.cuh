@@ -149,39 +149,48 @@ int step_pre_t(falm_ctx *ctx, const falm_fields *f, double dt, double t, cudaStr
     T *ua = (T *)ctx->w_ua, *rhs = (T *)ctx->w_rhs;
     const bool chan = ctx->bc_kind == FALM_BC_CHANNEL;
     bool fused_res = false;
-    // recording: the guide-shell copy (u -> ua) and, in a channel, the saved
-    // outlet velocity (u -> w_outlet, read by the velocity BC after the
-    // projection) depend only on the step's input velocity, so they run on a
-    // side branch beside the forcing and the pseudo-velocity, which write
-    // neither; the branch joins before the face-velocity pass reads ua
+    // 1. ALM (src/alm/alm.h:66-77) at the previous velocity, or the RMCP model; the
+    // ALM's force (a caller's field, or without one the force boxes) is added to the
+    // pseudo-velocity after it
+    const bool boxes = ctx->alm_on && !ff;
+    // recording: the force boxes, the guide-shell copy (u -> ua) and, in a channel,
+    // the saved outlet velocity (u -> w_outlet, read by the velocity BC after the
+    // projection) depend only on the step's input velocity, so they run on a side
+    // branch beside the pseudo-velocity, which reads none of them and writes other
+    // cells of ua; the branch joins before the force is added
     const bool side = t_dev && ctx->side_stream;
+    if (phase) phase->next("forcing");
     if (side) {
         const cudaStream_t ss = ctx->side_stream;
         CK(cudaEventRecord(ctx->side_fork, st));
         CK(cudaStreamWaitEvent(ss, ctx->side_fork, 0));
+        if (boxes && (rc = alm_run_t<T>(ctx, u, nullptr, t, ss, t_dev))) return rc;
         LAUNCH(FALM_K_OTHER, ss, k_copy_shell<T><<<ctx->sm_count * 8, 256, 0, ss>>>(g, u, ua));
         if (chan) { LAUNCH(FALM_K_OTHER, ss, k_save_outlet<T><<<std::min(ctx->sm_count * 4, (3 * g.sy * g.sz + 255) / 256), 256, 0, ss>>>(g, u, (T *)ctx->w_outlet)); }
         CK(cudaEventRecord(ctx->side_join, ss));
+    } else if (boxes && (rc = alm_run_t<T>(ctx, u, nullptr, t, st, t_dev))) {
+        return rc;
     }
-    // 1. ALM (src/alm/alm.h:66-77) at the previous velocity, or the RMCP model
-    if (phase) phase->next("forcing");
     if (ctx->alm_on) {
-        if ((rc = alm_run_t<T>(ctx, u, ff, t, st, t_dev))) return rc;
+        if (!boxes && (rc = alm_run_t<T>(ctx, u, ff, t, st, t_dev))) return rc;
     } else if (ctx->rmcp_on) {
         ff = (T *)ctx->w_ff;
         if ((rc = rmcp_run_t<T>(ctx, u, ff, nullptr, t, st, t_dev))) return rc;
     }
-    // 2. pseudo-velocity into ua (ALM force projected in-kernel when ff == NULL)
+    // 2. pseudo-velocity into ua
     if (phase) phase->next("pseudo_velocity");
-    if ((rc = pseudo_u_t<T>(ctx, u, u, uu, ua, nut, ff, dt, ctx->alm_on != 0, st))) return rc;
+    if ((rc = pseudo_u_t<T>(ctx, u, u, uu, ua, nut, ctx->alm_on ? nullptr : ff, dt, false, st))) return rc;
+    if (side) CK(cudaStreamWaitEvent(st, ctx->side_join, 0));
+    if (ctx->alm_on && ctx->alm.bs.total > 0)
+        LAUNCH(FALM_K_ALM, st, k_alm_add<T><<<(int)std::min<long long>((ctx->alm.bs.total + 255) / 256, (long long)ctx->sm_count * 8), 256, 0, st>>>(
+                                   g, ctx->alm, ua, ff, (T)dt));
     // 3. face velocity + [uubc] + RHS in one pass
     if (phase) phase->next("face_velocity_rhs");
     {
         const Region3 R = facemap(g);
         T scale = (T)(1.0 / (dt * ctx->maxdiag));
         // the guide layer of ua takes the previous velocity (the reference's aliased u)
-        if (side) CK(cudaStreamWaitEvent(st, ctx->side_join, 0));
-        else LAUNCH(FALM_K_OTHER, st, k_copy_shell<T><<<ctx->sm_count * 8, 256, 0, st>>>(g, u, ua));
+        if (!side) LAUNCH(FALM_K_OTHER, st, k_copy_shell<T><<<ctx->sm_count * 8, 256, 0, st>>>(g, u, ua));
         // the plane stream also computes the solve's first residual (rr) and
         // first preconditioner sweep (pp) from the pressure p, the initial guess
         fused_res = false;
@@ -317,7 +326,9 @@ int step_graph_t(falm_ctx *ctx, const falm_fields *f, double dt, double t, cudaS
     if (!sg) {
         if (!ctx->cap_stream) CK(cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
         if (!ctx->side_stream) {
-            CK(cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking));
+            int least = 0, most = 0;   // ahead of the pseudo-velocity's waiting blocks
+            CK(cudaDeviceGetStreamPriorityRange(&least, &most));
+            CK(cudaStreamCreateWithPriority(&ctx->side_stream, cudaStreamNonBlocking, most));
             CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
             CK(cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming));
         }
