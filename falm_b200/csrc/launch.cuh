@@ -421,7 +421,14 @@ int pc_mv_launch(falm_ctx *ctx, cudaStream_t st, const T *r, T *z) {
     v.a0 = (T *)ctx->w_p; v.b0 = (T *)ctx->w_q;
     v.a1 = (T *)ctx->w_s; v.b1 = (T *)ctx->w_t;
     v.z = z;
-    auto kern = pairs_ok(ctx, r, r) ? k_pc_mv<T, MODE, true> : k_pc_mv<T, MODE, false>;
+    const bool aln = pairs_ok(ctx, r, r);
+    auto kern = aln ? k_pc_mv<T, MODE, true, false> : k_pc_mv<T, MODE, false, false>;
+    // general z coefficients in FP64: half the divisions (an FP32 weight is one
+    // approximate reciprocal).  A run shorter than 16 planes leaves most chunks
+    // without an iteration of five regular planes.
+    if constexpr (sizeof(T) == 8) {
+        if (ctx->zrun1 - ctx->zrun0 < 16 && ctx->zrun1 - ctx->zrun0 < g.nz - 2) kern = aln ? k_pc_mv<T, MODE, true, true> : k_pc_mv<T, MODE, false, true>;
+    }
     constexpr int smem = L::template smem<MODE == 0 ? 3 : 2>();
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int bx = L::tiles_x(g.nx), by = L::tiles_y(g.ny);

@@ -42,7 +42,7 @@
 // Measured, s half at 512 x 256 x 256 (cold, one kernel at a time): FP32 update
 // 111 + sweeps 221 + product 107 -> 188 us, FP64 208 + 623 + 172 -> 348 us; FP64
 // iteration at 128 x 64 x 64 85 -> 64 us, at 200 x 120 x 96 (general z
-// coefficients) 260 -> 165 us.
+// coefficients) 260 -> 148 us.
 #pragma once
 #include "pair.cuh"
 #include "poisson.cuh"
@@ -85,8 +85,11 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // MODE 0: P, 1: S.  ALN: rows, bases and tile origins allow pair accesses.
-// [zr0, zr1): the longest run of planes with equal z coefficients.
-template <typename T, int MODE, bool ALN>
+// [zr0, zr1): the longest run of planes with equal z coefficients.  GEN (FP64, no
+// such run): a plane's weights, a division each, are computed when stages 0 and 1
+// reach it and kept for stages 2 and 3 two iterations later, on the same cells
+// (200 x 120 x 96 stretched: 168 -> 148 us an iteration).
+template <typename T, int MODE, bool ALN, bool GEN>
 __global__ void __launch_bounds__(PCTile<T>::NT, 1) k_pc_mv(Geom g, int kc, PoissonTables<T> tb, PCVec<T> vec, T omega, int zr0, int zr1,
                                                             RedWork rw, SolverScalars *sc) {
     using L = PCTile<T>;
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(PCTile<T>::NT, 1) k_pc_mv(Geom g, int kc, Pois
             wS[s] = mk2(inx[s] && iny[0] ? weight(acS[s].x) : T(0), inx[1 - s] && iny[1] ? weight(acS[s].y) : T(0));
         }
     }
-    if constexpr (L::CSM) {
+    if constexpr (L::CSM && !GEN) {
 #pragma unroll
         for (int s = 0; s < 2; s++) { scoef[s * NT + tid] = acS[s]; scoef[(2 + s) * NT + tid] = wS[s]; }
     }
@@ -233,6 +236,10 @@ __global__ void __launch_bounds__(PCTile<T>::NT, 1) k_pc_mv(Geom g, int kc, Pois
         }
     };
 
+    if constexpr (GEN) {   // the weights of stages 2 and 3, none yet
+#pragma unroll
+        for (int s = 0; s < 4; s++) scoef[s * NT + tid] = z2;
+    }
     // one iteration: plane q arrives (cell x0 of the first row at offset c); S its colour parity; REG: planes
     // q - 4 .. q have the regular z coefficients
     int slot = 0;   // of plane q
@@ -272,7 +279,11 @@ __global__ void __launch_bounds__(PCTile<T>::NT, 1) k_pc_mv(Geom g, int kc, Pois
                 ab[m] = mk2(zc.ab, zc.ab); at[m] = mk2(zc.at, zc.at); nat[m] = mk2(-zc.at, -zc.at);
                 ac[m] = mul2(add2(add2(dS, mk2(zc.nup, zc.nup)), mk2(zc.num, zc.num)), mk2(tb.scale, tb.scale));
                 const bool in = pl >= gc && pl < g.sz - gc;
-                if (m < 4) w[m] = mk2(in && inx[S] && iny[0] ? weight(ac[m].x) : T(0), in && inx[Q] && iny[1] ? weight(ac[m].y) : T(0));
+                if (m < (GEN ? 2 : 4)) w[m] = mk2(in && inx[S] && iny[0] ? weight(ac[m].x) : T(0), in && inx[Q] && iny[1] ? weight(ac[m].y) : T(0));
+            }
+            if constexpr (GEN) {
+                w[2] = scoef[S * NT + tid]; w[3] = scoef[(2 + S) * NT + tid];
+                scoef[S * NT + tid] = w[0]; scoef[(2 + S) * NT + tid] = w[1];
             }
         }
         __syncthreads();   // the planes the stages left at the previous iteration
@@ -377,10 +388,12 @@ __global__ void __launch_bounds__(PCTile<T>::NT, 1) k_pc_mv(Geom g, int kc, Pois
     using P1 = std::integral_constant<int, 1>;
     unsigned c = c00 + (unsigned)qs * sxy;
     for (int q = qs; q <= qe; q += 2, c += 2 * sxy) {
-        if (q - 4 >= zr0 && q + 1 < zr1) {
-            iter(P0{}, std::true_type{}, q, c);
-            if (q + 1 > qe) break;
-            iter(P1{}, std::true_type{}, q + 1, c + sxy);
+        if (!GEN && q - 4 >= zr0 && q + 1 < zr1) {
+            if constexpr (!GEN) {
+                iter(P0{}, std::true_type{}, q, c);
+                if (q + 1 > qe) break;
+                iter(P1{}, std::true_type{}, q + 1, c + sxy);
+            }
         } else {
             iter(P0{}, std::false_type{}, q, c);
             if (q + 1 > qe) break;
