@@ -252,13 +252,13 @@ def step_bytes(S, n, it, m=2):
 # each operand once): used for the per-kernel achieved bandwidth
 KERNEL_VALUES = {
     "pseudo_u": 10,     # u(3) uu(3) nut(1) in, ua(3) out (ALM force evaluated in-kernel)
-    "utouu_rhs": 10,    # ua(3) p(1) in, uu(3) rhs(1) rr(1) pp(1) out (the solve's first residual fused in)
+    "utouu_rhs": 9,     # ua(3) p(1) in, uu(3) rhs(1) rr(1) out (the solve's first residual fused in)
     "res": 2,           # the mixed-precision outer check: x b in (a pass residual after a failed check: 4)
     "bicg_p": 5,        # r p q in, p pp out (from a pass's second iteration on)
     "sor": 3,           # x b in, x out (three red-black half sweeps per launch, one HBM pass)
-    "mv_dot1": 3,       # pp rr in, q out
+    "mv_dot1": 3,       # the p half of an iteration: rr in, pp q out in a pass's first one (r p q rr in, p pp q out after)
     "bicg_s": 4,        # r q in, s ss out
-    "mv_dot2": 3,       # ss s in, t out
+    "mv_dot2": 5,       # the s half: r q in, s ss t out
     "bicg_xr": 8,       # x pp ss s t rr in, x r out
     "project": 13,      # ua(3) uu(3) p in, u(3) uu(3) out
     "sgs_div": 7,       # u(3) uu(3) in, nut out
