@@ -381,7 +381,15 @@ bool pc_first_in_xp(const falm_ctx *ctx) {
 
 // Whether the solver's iterations run as fused half iterations (pc_mv.cuh):
 // the drivers' preconditioner (red-black SOR, two sweeps) on the table operator.
+// Not in FP64 on grids of less than 2^17 cells whose rows TMA cannot address: the
+// separate kernels are row kernels there, of 4-5 us each, and a half iteration's
+// planes cost more (20 iterations, rows against fused: 41 x 31 x 30 1032 and 1122 us,
+// 75 x 41 x 40 1113 and 1170; at 63^3 the iteration's kernels 110 and 56, cold; in
+// FP32 1234 and 1070, 1319 and 1102).
+template <typename T>
 bool pc_half_ok(const falm_ctx *ctx) {
+    const Geom &g = ctx->geo;
+    if (sizeof(T) == 8 && ((g.sx * sizeof(T)) & 15) != 0 && (long long)g.nx * g.ny * g.nz < (1 << 17)) return false;
     return ctx->pc_type == FALM_LS_SOR && ctx->pc_maxit == 2 && !ctx->A_explicit && !ctx->no_tma && !ctx->sor_v1;
 }
 

@@ -277,7 +277,7 @@ int solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *it_out,
     // the stream of the iteration kernels: st, or the capture stream while a
     // device-side loop (CUDA graph) is recorded
     cudaStream_t ist = st;
-    const bool first_xp = pc_first_in_xp<T>(ctx), half = pc_half_ok(ctx);
+    const bool first_xp = pc_first_in_xp<T>(ctx), half = pc_half_ok<T>(ctx);
     auto first_target = [&](T *z) -> T * { return first_xp ? xp : z; };
     // launch the remaining sweeps of one preconditioner application z ~ A^-1 v
     // (the first, pointwise sweep wrote first_target(z)); the temporally blocked

@@ -203,7 +203,7 @@ int step_pre_t(falm_ctx *ctx, const falm_fields *f, double dt, double t, cudaStr
                 return rc;
             }
             const Op7<T> op = op7<T>(ctx);
-            T *ppt = pc_half_ok(ctx) ? nullptr : (pc_first_in_xp<T>(ctx) ? (T *)ctx->w_xp : (T *)ctx->w_pp);
+            T *ppt = pc_half_ok<T>(ctx) ? nullptr : (pc_first_in_xp<T>(ctx) ? (T *)ctx->w_xp : (T *)ctx->w_pp);
             const void *const fp[2] = {ua, p};
             const int nc[2] = {3, 1};
             int s3;
