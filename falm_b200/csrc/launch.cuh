@@ -379,18 +379,26 @@ bool pc_first_in_xp(const falm_ctx *ctx) {
     return (passes & 1) != 0;
 }
 
+// z planes per CTA of a half iteration, 0: more blocks than the reduction workspace holds
+template <typename T>
+int pc_planes(const falm_ctx *ctx) {
+    const Geom &g = ctx->geo;
+    return pc_chunk<T>(g.nx, g.ny, g.nz, ctx->sm_count, ctx->red.maxBlocks);
+}
+
 // Whether the solver's iterations run as fused half iterations (pc_mv.cuh):
 // the drivers' preconditioner (red-black SOR, two sweeps) on the table operator.
 // Not in FP64 on grids of less than 2^17 cells whose rows TMA cannot address: the
 // separate kernels are row kernels there, of 4-5 us each, and a half iteration's
 // planes cost more (20 iterations, rows against fused: 41 x 31 x 30 1032 and 1122 us,
 // 75 x 41 x 40 1113 and 1170; at 63^3 the iteration's kernels 110 and 56, cold; in
-// FP32 1234 and 1070, 1319 and 1102).
+// FP32 1234 and 1070, 1319 and 1102).  Nor where a block would have no slot for its
+// partial sums (pc_planes 0): the row kernels bound their own grids.
 template <typename T>
 bool pc_half_ok(const falm_ctx *ctx) {
     const Geom &g = ctx->geo;
     if (sizeof(T) == 8 && ((g.sx * sizeof(T)) & 15) != 0 && (long long)g.nx * g.ny * g.nz < (1 << 17)) return false;
-    return ctx->pc_type == FALM_LS_SOR && ctx->pc_maxit == 2 && !ctx->A_explicit && !ctx->no_tma && !ctx->sor_v1;
+    return ctx->pc_type == FALM_LS_SOR && ctx->pc_maxit == 2 && !ctx->A_explicit && !ctx->no_tma && !ctx->sor_v1 && pc_planes<T>(ctx) > 0;
 }
 
 // whether the interior's cells can be accessed in aligned pairs from the first
@@ -400,22 +408,6 @@ template <typename T>
 bool pairs_ok(const falm_ctx *ctx, const T *a, const T *b) {
     const Geom &g = ctx->geo;
     return ((g.gc | g.sx | g.nx) & 1) == 0 && (((uintptr_t)a | (uintptr_t)b) % (2 * sizeof(T))) == 0;
-}
-
-// z planes per CTA of a half iteration: the chunk that minimises waves x
-// (planes + the eight of the pipeline's fill + about six for the start and the
-// reduction); one CTA is resident per SM
-template <typename T>
-int pc_chunk(const falm_ctx *ctx, long long tiles, int nz) {
-    int best = 1;
-    long long best_t = -1;
-    for (int kc = std::min(nz, PCTile<T>::KMAX); kc >= std::min(nz, 2); kc--) {
-        const long long ctas = tiles * ((nz + kc - 1) / kc);
-        if (ctas > ctx->red.maxBlocks) break;
-        const long long t = ((ctas + ctx->sm_count - 1) / ctx->sm_count) * (kc + 2 * PCTile<T>::H + 6);
-        if (best_t < 0 || t < best_t) { best_t = t; best = kc; }
-    }
-    return best;
 }
 
 // one half iteration: MODE 0 the p half (z = pp), 1 the s half (z = ss)
@@ -440,7 +432,8 @@ int pc_mv_launch(falm_ctx *ctx, cudaStream_t st, const T *r, T *z) {
     constexpr int smem = L::template smem<MODE == 0 ? 3 : 2>();
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const int bx = L::tiles_x(g.nx), by = L::tiles_y(g.ny);
-    const int kc = pc_chunk<T>(ctx, (long long)bx * by, g.nz);
+    const int kc = pc_planes<T>(ctx);
+    if (kc <= 0) return fail(ctx, FALM_ERR_STATE, "half iteration: more blocks than the reduction workspace holds");
     const dim3 grid(bx, by, (g.nz + kc - 1) / kc);
     LAUNCH(MODE == 0 ? FALM_K_MV_DOT1 : FALM_K_MV_DOT2, st,
            kern<<<grid, L::NT, smem, st>>>(g, kc, op7<T>(ctx).t, v, (T)ctx->pc_relax, ctx->zrun0, ctx->zrun1, ctx->red, ctx->scal));

@@ -31,7 +31,7 @@
 // solver's vectors.  The tile's outer four cells are recomputed by the
 // neighbouring tiles: a tile of 64 x 32 (FP32) or 64 x 24 (FP64) cells owns
 // 56 x 24 or 56 x 16 (and up to the walls where it touches them).  Operands are
-// copied to shared memory four planes ahead by cp.async, each thread its own
+// copied to shared memory NS planes ahead (four in FP32, three in FP64) by cp.async, each thread its own
 // cells, so no alignment of the rows is needed: pairs of 8 or 16 bytes where the
 // rows allow it, single cells elsewhere.
 //
@@ -45,30 +45,11 @@
 // coefficients) 260 -> 148 us.
 #pragma once
 #include "pair.cuh"
+#include "pc_tile.cuh"
 #include "poisson.cuh"
 #include "sor_rb_tma.cuh"
 
 namespace fb {
-
-template <typename T>
-struct PCTile {
-    static constexpr int H = 4;                                   // halo: stages after the first
-    static constexpr int NW = sizeof(T) == 4 ? 16 : 12, NT = 32 * NW;
-    static constexpr int TX = 64, TY = 2 * NW, OX = TX - 2 * H, OY = TY - 2 * H;
-    static constexpr int NS = sizeof(T) == 4 ? 4 : 3;             // planes of the operand ring
-    // FP32: every stage with the operations of sor_point() and dot7p() in their order, so that an iterate has the bits of the
-    // stand-alone kernels (an FP32 recursion with restarts is sensitive to a consistent operator: sharing stage 3's sum with
-    // the product, as FP64 does, left the same error per application but 4 times the error after five restarts)
-    static constexpr bool SEQ = sizeof(T) == 4;
-    static constexpr bool CSM = sizeof(T) == 8;                   // the cells' diagonals and weights kept in shared memory (registers are full)
-    static constexpr int XP = TX / 2 + 2, EPL = (TY + 2) * XP;    // a stage's plane: pairs and rows with a border
-    static constexpr int KMAX = 96, ZPL = KMAX + 2 * H + 8;       // planes of a chunk; staged z coefficients
-    template <int NF> static constexpr int smem() {
-        return (NS * NF * 2 * NT * 2 + 8 * EPL + 4 * ZPL + 4 * NT + (CSM ? 8 * NT : 0)) * (int)sizeof(T);
-    }
-    static int tiles_x(int n) { return n <= TX ? 1 : (n - 2 * H + OX - 1) / OX; }
-    static int tiles_y(int n) { return n <= TY ? 1 : (n - 2 * H + OY - 1) / OY; }
-};
 
 // The vectors of an iteration.  The new p and q may not overwrite the old ones,
 // which neighbouring tiles still read, so {p, q} and {s, t} change places at
