@@ -444,9 +444,9 @@ int pc_mv_launch(falm_ctx *ctx, cudaStream_t st, const T *r, T *z) {
 // cannot (BoxCopy): two guide cells on every side, as the boxes' halos assume.
 // Before, such grids ran the row kernels, which recompute the metric of every
 // neighbour and read every neighbour through L1: the pseudo-velocity of the
-// 301 x 157 x 131 channel 387 us in FP32 (180 copied), face velocity + residual
-// 72 + 85 (108), the check 85 (46), SGS 118 (103), projection 83 (69); in FP64 861
-// (242), 126 + 114 (139), SGS 207 (147), projection 157 (119).  A body's kMinCopied:
+// 301 x 157 x 131 channel 387 us in FP32 (186 copied), face velocity + residual
+// 72 + 85 (112), the check 85 (46), SGS 118 (103), projection 83 (69); in FP64 861
+// (246), 126 + 114 (148), SGS 207 (135), projection 157 (119).  A body's kMinCopied:
 // cells below which its row kernel is the faster one, on small grids where a plane
 // stream is bound by the latency of its planes (63^3: SGS 13 us against 20,
 // projection 6 against 12; 101^3: equal within 15% either way).

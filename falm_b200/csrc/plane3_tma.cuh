@@ -45,8 +45,16 @@ struct P3View {
 };
 
 // metric factors of the 3 x 3 columns around (i, j) and of planes k-1..k+1, with
-// MetricView's association (ja = (hx*hy)*hz, g_d = (ja*k_d)*k_d); offsets -1, 0, +1
-template <typename T>
+// MetricView's association (ja = (hx*hy)*hz, g_d = (ja*k_d)*k_d); offsets -1, 0, +1.
+// QUOT: the volume itself is divided by and its cube root taken, as the row kernels
+// do, in place of products of the inverse widths and of the widths' cube roots.  The
+// face velocity carries the rounded volume as a factor, which only a division by the
+// same volume cancels: on grids whose widths and inverse widths round to different
+// sides the product left the pressure of an FP32 step with 1.6 times the row
+// kernels' error (63^3: 7.0e-7 and 4.3e-7), and the rounded cube roots the eddy
+// viscosity with 1.4 times (185 x 91 x 87: 4.5e-7 and 3.2e-7).  It is set on copied
+// boxes, which took the row kernels' place on their grids.
+template <typename T, bool QUOT>
 struct ColMet {
     T hx[3], kx[3], hy[3], ky[3], hz[3], kz[3];
     __device__ __forceinline__ T ja(int dx, int dy, int dz) const { return (hx[1 + dx] * hy[1 + dy]) * hz[1 + dz]; }
@@ -54,6 +62,15 @@ struct ColMet {
     __device__ __forceinline__ T g(int d, int dx, int dy, int dz) const {
         const T kk = k(d, dx, dy, dz);
         return (ja(dx, dy, dz) * kk) * kk;
+    }
+    // v / ja of the cell, and the filter width (cxy and cz: cube roots of hx hy and hz)
+    __device__ __forceinline__ T over_ja(T v) const {
+        if constexpr (QUOT) return v / ja(0, 0, 0);
+        else return v * ((kx[1] * ky[1]) * kz[1]);
+    }
+    __device__ __forceinline__ T width(T cxy, T cz) const {
+        if constexpr (QUOT) return cbrt(ja(0, 0, 0));
+        else return cxy * cz;
     }
 };
 
@@ -126,7 +143,7 @@ __global__ void __launch_bounds__(256, (p3_minb<T, Body>())) k_plane3_tma(Geom g
 #pragma unroll
     for (int d = 0; d < (NV > 0 ? NV : 1); d++) acc[d] = 0.0;
     // column metric factors (x shared by the rows, y per row); z rolled per plane below
-    ColMet<T> cm[RY];
+    ColMet<T, CPA> cm[RY];
     typename Body::CS cst[RY];
 #pragma unroll
     for (int r = 0; r < RY; r++) cst[r] = body.col_state(min(i, R.i1 - 1), min(jr[r], R.j1 - 1));
@@ -279,7 +296,8 @@ struct UtoUUBody {
     __device__ PW pw_load(int, int, int, long long) const { return PW{}; }
     __device__ CS col_state(int, int) const { return CS{}; }
     __device__ ZS plane_state(int) const { return ZS{}; }
-    __device__ __forceinline__ T ucv(const P3View<T, 1> &v, const ColMet<T> &cm, int d, int dx, int dy, int dz) const {
+    template <class CM>
+    __device__ __forceinline__ T ucv(const P3View<T, 1> &v, const CM &cm, int d, int dx, int dy, int dz) const {
         return cm.ja(dx, dy, dz) * cm.k(d, dx, dy, dz) * v.at(0, d, dz, dx, dy);
     }
     __device__ __forceinline__ bool zero_face(int d, int i, int j, int k) const {
@@ -290,21 +308,22 @@ struct UtoUUBody {
         return ((k == g.gc - 1 && (g.zphys & 1)) || (k == g.sz - g.gc - 1 && (g.zphys & 2))) && iin && jin;   // not at slab interfaces
     }
     // face d of cell (i+dx, j+dy, k+dz) (the face towards +d)
-    __device__ __forceinline__ T face(const P3View<T, 1> &v, const ColMet<T> &cm, int d, int i, int j, int k, int dx, int dy,
+    template <class CM>
+    __device__ __forceinline__ T face(const P3View<T, 1> &v, const CM &cm, int d, int i, int j, int k, int dx, int dy,
                                       int dz) const {
         if (zero_face(d, i + dx, j + dy, k + dz)) return T(0);
         T a = ucv(v, cm, d, dx, dy, dz);
         T b = ucv(v, cm, d, dx + (d == 0), dy + (d == 1), dz + (d == 2));
         return T(0.5) * (a + b);
     }
-    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 1> &v, const ColMet<T> &cm, const PW &, const CS &,
+    template <class CM>
+    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 1> &v, const CM &cm, const PW &, const CS &,
                          const ZS &, double (&)[1]) const {
         const T UE = face(v, cm, 0, i, j, k, 0, 0, 0), VN = face(v, cm, 1, i, j, k, 0, 0, 0), WT = face(v, cm, 2, i, j, k, 0, 0, 0);
         uu[c] = UE; uu[c + g.n] = VN; uu[c + 2 * g.n] = WT;
         if (RHS && i >= g.gc && j >= g.gc && k >= g.gc) {
             const T UW = face(v, cm, 0, i, j, k, -1, 0, 0), VS = face(v, cm, 1, i, j, k, 0, -1, 0), WB = face(v, cm, 2, i, j, k, 0, 0, -1);
-            // 1/ja as the product of the inverse widths
-            T div = (UE - UW + VN - VS + WT - WB) * ((cm.kx[1] * cm.ky[1]) * cm.kz[1]);
+            T div = cm.over_ja(UE - UW + VN - VS + WT - WB);
             rhs[c] = div * scale;
         }
     }
@@ -341,7 +360,8 @@ struct ProjectBody {
         if (i >= g.gc && j >= g.gc && k >= g.gc) { w.a0 = ua[cc]; w.a1 = ua[cc + N]; w.a2 = ua[cc + 2 * N]; }
         return w;
     }
-    __device__ void cell(int i, int j, int k, long long cc, const P3View<T, 1> &v, const ColMet<T> &cm, const PW &w, const CS &,
+    template <class CM>
+    __device__ void cell(int i, int j, int k, long long cc, const P3View<T, 1> &v, const CM &cm, const PW &w, const CS &,
                          const ZS &, double (&)[1]) const {
         const long long N = g.n;
         const T pcc = v.at(0, 0, 0), pe = v.at(0, 0, 0, 1, 0), pn = v.at(0, 0, 0, 0, 1), pt = v.at(0, 0, 1);
@@ -388,7 +408,8 @@ struct UtoUUResBody {
     __device__ PW pw_load(int, int, int, long long) const { return PW{}; }
     __device__ CS col_state(int i, int j) const { return op.column(i, j); }
     __device__ ZS plane_state(int k) const { return op.zplane(k); }
-    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 2> &v, const ColMet<T> &cm, const PW &, const CS &cs,
+    template <class CM>
+    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 2> &v, const CM &cm, const PW &, const CS &cs,
                          const ZS &zs, double (&acc)[2]) const {
         const Geom &g = uub.g;
         // the face velocity and, at interior cells, the RHS (UtoUUBody's expressions)
@@ -401,7 +422,7 @@ struct UtoUUResBody {
         if (i >= g.gc && j >= g.gc && k >= g.gc) {
             const T UW = uub.face(v1, cm, 0, i, j, k, -1, 0, 0), VS = uub.face(v1, cm, 1, i, j, k, 0, -1, 0),
                     WB = uub.face(v1, cm, 2, i, j, k, 0, 0, -1);
-            const T div = (UE - UW + VN - VS + WT - WB) * ((cm.kx[1] * cm.ky[1]) * cm.kz[1]);
+            const T div = cm.over_ja(UE - UW + VN - VS + WT - WB);
             const T bv = div * uub.scale;
             uub.rhs[c] = bv;
             // r = b - A p in FP64, the 7-point products accumulated in ResBody's order
@@ -457,7 +478,8 @@ struct P3ResBody {
     __device__ PW pw_load(int, int, int, long long c) const { return PW{rb.b[c]}; }
     __device__ CS col_state(int i, int j) const { return rb.op.column(i, j); }
     __device__ ZS plane_state(int k) const { return rb.op.zplane(k); }
-    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 1> &v, const ColMet<T> &, const PW &w, const CS &cs, const ZS &zs,
+    template <class CM>
+    __device__ void cell(int i, int j, int k, long long c, const P3View<T, 1> &v, const CM &, const PW &w, const CS &cs, const ZS &zs,
                          double (&acc)[ResBody<T, CHECK>::NV]) const {
         const T ac = rb.op.ac_col(cs, zs);
         double ax = (double)ac * (double)v.at(0, 0, 0);
@@ -506,8 +528,8 @@ struct SgsDivBody {
         return CS{cbrt(ldg(mv.m.h[0] + i)) * cbrt(ldg(mv.m.h[1] + j)), ldg(m64.k[0] + i) * ldg(m64.k[1] + j)};
     }
     __device__ ZS plane_state(int k) const { return ZS{cbrt(ldg(mv.m.h[2] + k)), ldg(m64.k[2] + k)}; }
-    template <int RYV>
-    __device__ void cell(int i, int j, int k, long long cc, const P3View<T, 2, RYV> &v, const ColMet<T> &cm, const PW &, const CS &cs,
+    template <int RYV, class CM>
+    __device__ void cell(int i, int j, int k, long long cc, const P3View<T, 2, RYV> &v, const CM &cm, const PW &, const CS &cs,
                          const ZS &zs, double (&acc)[1]) const {
         if (sgs != FALM_SGS_EMPTY) {
             const T kxx = cm.kx[1], kxy = cm.ky[1], kxz = cm.kz[1];
@@ -524,7 +546,7 @@ struct SgsDivBody {
             T d1 = T(2) * (dux * dux), d2 = T(2) * (dvy * dvy), d3 = T(2) * (dwz * dwz);
             T d4 = (duy + dvx) * (duy + dvx), d5 = (dvz + dwy) * (dvz + dwy), d6 = (duz + dwx) * (duz + dwx);
             T Du = sqrt(d1 + d2 + d3 + d4 + d5 + d6);
-            T De = cs.cbxy * zs.cbz;
+            T De = cm.width(cs.cbxy, zs.cbz);
             if (sgs == FALM_SGS_SMAGORINSKY) {
                 T lc = Cs * De;
                 nut[cc] = (lc * lc) * Du;

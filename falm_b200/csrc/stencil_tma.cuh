@@ -131,7 +131,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
     // The face factors g_d(c) + g_d(c+-e_d) of the diffusion, g_d = ja k_d^2 and
     // ja = hx hy hz, separate: an x/y face's is hz times a column constant, a z
     // face's is hx hy times a plane constant (the reference's values up to
-    // rounding); 1/ja is the product of the inverse widths.
+    // rounding); 1/ja is the product of the inverse widths, but on copied boxes the
+    // reciprocal of the volume itself (ColMet's QUOT).
     const T kxc2 = kxc * kxc, kyc2 = kyc * kyc;
     const T Axe = Pc * kxc2 + Pe * (kxe * kxe), Axw = Pc * kxc2 + Pw * (kxw * kxw);
     const T Ayn = Pc * kyc2 + Pn * (kyn * kyn), Ays = Pc * kyc2 + Ps * (kys * kys);
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 3) k_pseudo_u_tma(Ge
             const T hzkz2 = hzk * (kzk * kzk);
             const T Bzt = hzkz2 + hzt * (kzt * kzt), Bzb = hzkz2 + hzb * (kzb * kzb);
             // the scheme's divisions by the Jacobian become multiplications by 1/ja
-            const T ij = kxy * kzk;
+            const T ij = CPA ? T(1) / (Pc * hzk) : kxy * kzk;
             const T UE = UU0[o], UW = UU0[o - 1], VN = UU0[L::PE + o], VS = UU0[L::PE + o - L::BX];
             const T WT = UU0[2 * L::PE + o], WB = uu2m1;
             const T nutcc = N0[o];

@@ -271,6 +271,77 @@ def test_copied_boxes_match_row_kernels(lib_built, monkeypatch, precision, pc, s
         assert rel_l2(outs[1][k], outs[0][k]) < tol[k], (k, rel_l2(outs[1][k], outs[0][k]))
 
 
+def _smooth_velocity(grid, seed):
+    """a few plane waves of random direction, amplitude 0.1 about a mean of 1, as FP32 values"""
+    rng = np.random.default_rng(seed)
+    z, y, x = np.meshgrid(grid.z, grid.y, grid.x, indexing="ij")
+    u = np.zeros((3, grid.sz, grid.sy, grid.sx))
+    u[0] = 1.0
+    for c in range(3):
+        for _ in range(4):
+            k = rng.integers(1, 5, 3) * 2 * np.pi / np.array([grid.sx * grid.hx[2], grid.sy * grid.hy[2], grid.sz * grid.hz[2]])
+            u[c] += 0.1 * np.sin(k[0] * x + k[1] * y + k[2] * z + rng.uniform(0, 2 * np.pi))
+    return u.astype(np.float32).astype(np.float64).ravel()
+
+
+@pytest.mark.parametrize("n", [55, 63, 83, 97, 125])
+def test_copied_boxes_round_as_the_row_kernels(lib_built, monkeypatch, n):
+    """Rows that TMA cannot address, FP32: the streams with copied boxes are as close
+    to the FP64 results from the same FP32 velocity as the row kernels are, on grids
+    where FP32 widths and inverse widths round to different sides (63, 125) and not:
+    the tendency of the pseudo-velocity (un = 0, dt = 1) from the face velocity of the
+    same context, and the fields of a step with one solver iteration, whose pressure
+    is as exact as the right-hand side.  Bound: the two round differently in every
+    operation, so 1.1 times the row kernels' error and 5e-9 (a tenth of FP32
+    rounding); where products of inverse widths took the place of a division by the
+    volume the tendency's error was 1.46 times theirs at 63, and the pressure's 1.64
+    times at 63 and 1.37 times at 125."""
+    case = cases.cavity(n)
+    g = case.grid
+    u0 = _smooth_velocity(g, n)
+
+    def run(precision):
+        ctx = make_ctx(case, precision)
+        ctx.eq_init(1, 1.0, case.pc, case.pc_maxit, case.pc_relax)
+        u, uu, p, nut = dev(ctx, u0), ctx.field(3), ctx.field(1), ctx.field(1)
+        ctx.utouu(u, uu)
+        ctx.sgs(u, nut)
+        out = {"nut": interior(host(nut), g)}
+        tend, zero = ctx.field(3), ctx.field(3)
+        ctx.pseudo_u(zero, u, uu, tend, nut, zero, 1.0)
+        out["tendency"] = interior(host(tend), g, 3)
+        ctx.step(u, uu, p, nut, None, case.dt, case.dt)
+        return dict(out, u=interior(host(u), g, 3), uu=faces(host(uu), g), p=interior(host(p), g), nut1=interior(host(nut), g))
+
+    exact = run("fp64")
+    monkeypatch.setenv("FALM_B200_NO_TMA", "1")
+    row = run("mixed")
+    monkeypatch.setenv("FALM_B200_NO_TMA", "0")
+    copied = run("mixed")
+    for k in exact:
+        e, r = rel_l2(copied[k], exact[k]), rel_l2(row[k], exact[k])
+        assert e < 1.1 * r + 5e-9, (k, e, r)
+
+
+@pytest.mark.parametrize("shape", [(129, 91, 91), (185, 91, 87)])
+def test_copied_sgs_rounds_as_the_row_kernel(lib_built, monkeypatch, shape):
+    """The eddy viscosity from FP32 velocities on 2^20 cells and more of width 0.05,
+    rows that TMA cannot address: as close to FP64 as the row kernel's (the product
+    of rounded cube roots in its filter width: 1.4 times its error)."""
+    case = cases.small_channel(*shape, intensity=0.0)
+    case.alm, case.grid = None, cases.uniform_grid(*shape, 0.05)
+    g = case.grid
+    u0 = _smooth_velocity(g, 5)
+    out = []
+    for precision, no_tma in (("fp64", "1"), ("mixed", "1"), ("mixed", "0")):
+        monkeypatch.setenv("FALM_B200_NO_TMA", no_tma)
+        ctx = make_ctx(case, precision)
+        nut = ctx.field(1)
+        ctx.sgs(dev(ctx, u0), nut)
+        out.append(interior(host(nut), g))
+    assert rel_l2(out[2], out[0]) < 1.1 * rel_l2(out[1], out[0])
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_snapshots_and_time_average(lib_built, tmp_path, precision):
     """Snapshot files queued during steps (more than the two staging buffers)
