@@ -11,7 +11,7 @@ struct PCTile {
     static constexpr int TX = 64, TY = 2 * NW, OX = TX - 2 * H, OY = TY - 2 * H;
     static constexpr int NS = sizeof(T) == 4 ? 4 : 3;             // planes of the operand ring
     // FP32: every stage with the operations of sor_point() and dot7p() in their order, so that an iterate has the bits of the
-    // stand-alone kernels (an FP32 recursion with restarts is sensitive to a consistent operator: sharing stage 3's sum with
+    // stand-alone stream kernels (an FP32 recursion with restarts is sensitive to a consistent operator: sharing stage 3's sum with
     // the product, as FP64 does, left the same error per application but 4 times the error after five restarts)
     static constexpr bool SEQ = sizeof(T) == 4;
     static constexpr bool CSM = sizeof(T) == 8;                   // the cells' diagonals and weights kept in shared memory (registers are full)

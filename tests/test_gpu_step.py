@@ -53,8 +53,8 @@ def small_cases():
     cav.tol = 1e-10
     # wide enough (nx >= 64) for every plane stream, including the 7-point one
     wide = cases.small_channel(72, 20, 16, intensity=0.05).with_inflow(nb=8)
-    # an odd interior width: rows whose pitch is not a multiple of 16 bytes,
-    # so every plane stream gives way to the row kernels
+    # an odd interior width: rows whose pitch is not a multiple of 16 bytes, so the
+    # plane streams' boxes are copied or give way to the row kernels
     odd = cases.small_channel(33, 19, 15, intensity=0.05).with_inflow(nb=8)
     return {"channel": ch, "cavity": cav, "wide": wide, "odd": odd}
 
@@ -125,12 +125,46 @@ def test_step_fp64_converged(oracle, lib_built, name):
 
 
 def test_step_alm_fused_equals_stored_force(lib_built):
-    """The in-kernel ALM projection and the stored ff field give the same step."""
+    """The force boxes and a stored force field, each added to the pseudo-velocity over
+    the boxes' cells, give the same step (test_step_three_rotors has the oracle)."""
     case = small_cases()["channel"]
     a, sa, _ = run_gpu(case, 3, fuse_alm=True)
     b, sb, _ = run_gpu(case, 3, fuse_alm=False)
     for k in a:
         assert rel_l2(a[k], b[k]) < 1e-13, k
+
+
+def _three_rotors(h, size, n_ap=6):
+    """three rotors of radius 1 whose force boxes overlap and are cut by the walls:
+    one fixed, one turning the other way, one on a pitching platform"""
+    one = cases.make_rotor((0.0, 0.0, 0.0), h, n_ap_per_blade=n_ap, eps_cells=1.0)
+    base = np.array([[0.30 * size[0], 0.45 * size[1], 0.50 * size[2]], [0.42 * size[0], 0.60 * size[1], 0.50 * size[2]],
+                     [0.75 * size[0], 0.40 * size[1], 0.45 * size[2]]])
+    hub = np.array([[0.0, 0.0, 0.0], [-0.1, 0.0, 0.2], [0.0, 0.0, 0.3]])
+    motion = np.array([[0.0, 0.0, 0.0], [0.0, 0.0, 0.0], [0.05, 3.0, 0.4]])
+    aps = cases.build_aps_py(one.stations, 9 * n_ap, n_ap, 1.0, 0.0)
+    return cases.AlmSetup(3, 3, n_ap, 1.0, 0.0, one.euler_eps, base, hub, np.array([7.0, -6.0, 8.0]), motion,
+                          np.array([0, 0, 2], dtype=np.int32), one.stations, aps, 1.0)
+
+
+@pytest.mark.parametrize("stored", [False, True])
+@pytest.mark.parametrize("graph", ["1", "0"])
+def test_step_three_rotors(oracle, lib_built, monkeypatch, graph, stored):
+    """Several turbines with overlapping force boxes, of which a cell takes the first
+    one's force only, from the boxes and from a stored field, recorded and host-driven,
+    against the oracle: fields, and every turbine's own torque and thrust."""
+    monkeypatch.setenv("FALM_B200_GRAPH", graph)
+    case = cases.small_channel(48, 28, 24, intensity=0.05).with_inflow(nb=8)
+    h = float(case.grid.hx[2])
+    case.alm = _three_rotors(h, (48 * h, 28 * h, 24 * h))
+    ref, rs = run_oracle(oracle, case, 4, maxit=6, tol=0.0)
+    got, gs, _ = run_gpu(case, 4, fuse_alm=not stored, maxit=6, tol=0.0)
+    for k, v in compare(case, got, ref).items():
+        assert v < 1e-10, (k, v)
+    for a, b in zip(gs, rs):
+        assert len(a["torque"]) == 3 and len(set(a["torque"])) == 3
+        for x, y in zip(a["torque"] + a["thrust"], list(b["torque"]) + list(b["thrust"])):
+            assert x == pytest.approx(y, rel=1e-10)
 
 
 def test_step_mixed_vs_fp64_oracle(oracle, lib_built):
