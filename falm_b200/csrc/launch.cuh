@@ -388,16 +388,18 @@ int pc_planes(const falm_ctx *ctx) {
 
 // Whether the solver's iterations run as fused half iterations (pc_mv.cuh):
 // the drivers' preconditioner (red-black SOR, two sweeps) on the table operator.
-// Not in FP64 on grids of less than 2^17 cells whose rows TMA cannot address: the
-// separate kernels are row kernels there, of 4-5 us each, and a half iteration's
-// planes cost more (20 iterations, rows against fused: 41 x 31 x 30 1032 and 1122 us,
-// 75 x 41 x 40 1113 and 1170; at 63^3 the iteration's kernels 110 and 56, cold; in
-// FP32 1234 and 1070, 1319 and 1102).  Nor where a block would have no slot for its
-// partial sums (pc_planes 0): the row kernels bound their own grids.
+// Not in FP64 on grids of less than 2^17 cells where the separate kernels are row
+// kernels, of 4-5 us each (rows that TMA cannot address or that are shorter than a
+// box): a half iteration's planes cost more there.  FP64 solves of 10 iterations in
+// us, rows against fused: 16^3 413 and 559, 32^3 421 and 569, 32 x 60 x 60 577 and
+// 580, 32 x 66 x 66 617 and 594, 51^3 780 and 619, 65 x 65 x 33 605 and 611; of 20
+// iterations 41 x 31 x 30 1032 and 1122, 75 x 41 x 40 1113 and 1170.  In FP32 the
+// fused ones win (33^3, 20 iterations: 1148 and 1071).  Nor where a block would have
+// no slot for its partial sums (pc_planes 0): the row kernels bound their own grids.
 template <typename T>
 bool pc_half_ok(const falm_ctx *ctx) {
     const Geom &g = ctx->geo;
-    if (sizeof(T) == 8 && ((g.sx * sizeof(T)) & 15) != 0 && (long long)g.nx * g.ny * g.nz < (1 << 17)) return false;
+    if (sizeof(T) == 8 && !sor_pass_ok<T>(ctx, 3) && (long long)g.nx * g.ny * g.nz < (1 << 17)) return false;
     return ctx->pc_type == FALM_LS_SOR && ctx->pc_maxit == 2 && !ctx->A_explicit && !ctx->no_tma && !ctx->sor_v1 && pc_planes<T>(ctx) > 0;
 }
 

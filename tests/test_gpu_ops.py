@@ -265,9 +265,16 @@ def test_blocked_sor_tiles_agree(lib_built, monkeypatch, shape, precision):
         np.testing.assert_array_equal(outs[0], other)
 
 
-# odd widths of 2^17 cells and more last: below, FP64 rows that TMA cannot address keep the row kernels
+# odd and narrow widths of 2^17 cells and more last: below, FP64 keeps the row kernels there
 HALF_SHAPES = [(3, 2, 2), (40, 20, 3), (57, 25, 12), (64, 32, 1), (65, 24, 9), (66, 33, 30), (120, 56, 5), (121, 41, 17), (180, 63, 11),
-               (121, 57, 20), (57, 25, 93), (67, 65, 33)]
+               (121, 57, 20), (57, 25, 93), (67, 65, 33), (3, 210, 210), (2, 257, 257), (30, 66, 67), (400, 2, 165)]
+
+
+def _fuses(grid, precision):
+    """where the half iterations run: FP64 keeps the row kernels on grids of less than
+    2^17 cells whose rows a TMA box of 40 x 14 cannot take"""
+    row_kernels = grid.sx % 2 or grid.sx < 40 or grid.sy < 14 or grid.gc != 2
+    return precision == "mixed" or not row_kernels or grid.n_interior >= 1 << 17
 
 
 def _solves_fused(ctx, *vectors):
@@ -307,8 +314,7 @@ def test_half_iterations_match_separate_kernels(lib_built, monkeypatch, shape, p
     """The fused half iterations (tiles of 64 x 32 or 64 x 24 cells that own 56 x 24
     or 56 x 16, up to the walls where they touch them; pairs or, at odd widths, single
     cells; regular and general z coefficients) against the row kernels, around the tile
-    sizes.  The kernels that run are checked: FP64 keeps the row kernels at odd widths
-    of less than 2^17 cells.  FP64: three iterations to rounding, 1e-12 over the
+    sizes.  The kernels that run are checked.  FP64: three iterations to rounding, 1e-12 over the
     growth of three iterations on these grids (below 50).  Mixed: two iterations a
     pass from the same FP32 data, FP32 rounding (6e-8) over the same growth and five
     passes."""
@@ -324,7 +330,7 @@ def test_half_iterations_match_separate_kernels(lib_built, monkeypatch, shape, p
         ctx.solve(xd, bd, rd)
         outs.append(interior(host(xd), g).copy())
         fused.append(_solves_fused(ctx, xd, bd, rd))
-    assert fused == [precision == "mixed" or nx % 2 == 0 or nx * ny * nz >= 1 << 17, False]
+    assert fused == [_fuses(g, precision), False]
     assert np.isfinite(outs[0]).all()
     assert rel_l2(outs[0], outs[1]) < HALF_TOL[precision]
 
@@ -358,7 +364,7 @@ def test_half_iterations_on_vectors_off_pair_alignment(lib_built, shape, precisi
 def test_half_iterations_with_more_guide_cells(lib_built, monkeypatch, gc, precision):
     """Three (odd rows of guide cells: single cells) and four guide cells: the other
     streams give way to the row kernels, the half iterations run; bound as above."""
-    case = _half_case(cases.uniform_grid(66, 33, 30, 0.05, gc=gc), precision)
+    case = _half_case(cases.uniform_grid(66, 65, 33, 0.05, gc=gc), precision)
     g = case.grid
     b, x0 = _half_data(g)
     outs = []
