@@ -242,37 +242,63 @@ def peaks():
 
 
 # ---------------------------------------------------------------- algorithmic bytes
-def step_bytes(S, n, it, m=2):
-    """bytes per step: S*N*[44 + it*(28 + 6m)] (4 B/value mixed, 8 B FP64); the ALM
-    support term 3*S*N_box is negligible against N and left out"""
-    return S * n * (44 + it * (28 + 6 * m))
-
-
 # values moved per interior cell by one launch of each kernel class (reads + writes,
-# each operand once): used for the per-kernel achieved bandwidth
+# each operand once)
 KERNEL_VALUES = {
-    "pseudo_u": 10,     # u(3) uu(3) nut(1) in, ua(3) out (ALM force evaluated in-kernel)
+    "pseudo_u": 10,     # u(3) uu(3) nut(1) in, ua(3) out
     "utouu_rhs": 9,     # ua(3) p(1) in, uu(3) rhs(1) rr(1) out (the solve's first residual fused in)
-    "res": 2,           # the mixed-precision outer check: x b in (a pass residual after a failed check: 4)
-    "bicg_p": 5,        # r p q in, p pp out (from a pass's second iteration on)
-    "sor": 3,           # x b in, x out (three red-black half sweeps per launch, one HBM pass)
-    "mv_dot1": 3,       # the p half of an iteration: rr in, pp q out in a pass's first one (r p q rr in, p pp q out after)
-    "bicg_s": 4,        # r q in, s ss out
+    "res": 2,           # the mixed-precision outer check: x b in
+    "res_pass": 3,      # class res too, the residual of a pass after a failed check: x b in, rr out
+    "mv_dot1": 7,       # the p half of an iteration: r p q rr in, p pp q out
+    "mv_dot1_first": 3,  # the same in a pass's first iteration: rr in, pp q out
     "mv_dot2": 5,       # the s half: r q in, s ss t out
     "bicg_xr": 8,       # x pp ss s t rr in, x r out
     "project": 13,      # ua(3) uu(3) p in, u(3) uu(3) out
     "sgs_div": 7,       # u(3) uu(3) in, nut out
 }
+STEP_CLASSES = ("pseudo_u", "utouu_rhs", "project", "sgs_div")
 
 
-def traffic_for(kernel):
-    """dram bytes per launch from the committed ncu summary, if one exists"""
+def class_launches(stats, mixed):
+    """launches with work of every entry of KERNEL_VALUES over the steps of `stats`, with
+    the drivers' preconditioner (the half iterations); a step's passes start at iteration
+    0 each, and in mixed precision each is followed by a check"""
+    its, passes = sum(x["it"] for x in stats), sum(max(1, x["outer"]) for x in stats)
+    c = {k: len(stats) for k in STEP_CLASSES}
+    first = min(its, passes)
+    c.update(mv_dot1=its - first, mv_dot1_first=first, mv_dot2=its, bicg_xr=its,
+             res=passes if mixed else 0, res_pass=passes - len(stats))
+    return c
+
+
+def class_traffic(cls, count, S, n):
+    """mean DRAM bytes a launch of the class from the committed ncu summary (None without
+    one of this grid and precision)"""
     path = os.path.join(ROOT, "profiles", "traffic.json")
     try:
         with open(path) as f:
-            return json.load(f).get(kernel)
+            d = json.load(f)
+        if (d["value_bytes"], d["cells"]) != (S, n):
+            return None
+        parts = [k for k in (cls, cls + "_first", cls + "_pass") if count.get(k)]
+        return sum(d[k] * count[k] for k in parts) / sum(count[k] for k in parts)
     except Exception:
         return None
+
+
+def step_bytes(S, n, stats):
+    """bytes the kernels of a step cannot do without, each operand read and each result
+    written once per launch (mean over `stats`; S = 4 B a value mixed, 8 B FP64); the
+    force boxes are negligible against n and left out"""
+    c = class_launches(stats, S == 4)
+    return S * n * sum(KERNEL_VALUES[k] * c[k] for k in c) / len(stats)
+
+
+def separate_pass_bytes(S, n, it, m=2):
+    """bytes per step by the convention in which every stage of an iteration is a pass of
+    its own: S*N*[44 + it*(28 + 6m)]; the fused iteration moves half of it, so a rate by
+    this count can exceed the memory's"""
+    return S * n * (44 + it * (28 + 6 * m))
 
 
 # ---------------------------------------------------------------- workload
@@ -347,10 +373,12 @@ def run_ours(args, rank, world, local):
         ms, st, _, _ = timed(sim, K)
         ms = max_over_ranks(ms, world)
         its = [x["it"] for x in st]
-        sb = step_bytes(4 if prec == "mixed" else 8, n, sum(its) / len(its))
+        S = 4 if prec == "mixed" else 8
+        per_s = lambda nbytes: nbytes / (ms / K / 1e3) / 1e9 / peak  # noqa: E731
         res = {"value": replica_rate(world, n, K, ms), "ms_per_step": ms / K, "steps_per_s": 1e3 * K / ms,
                "its": it_summary(its), "outer_max": max(x["outer"] for x in st),
-               "divnorm_max": max(x["divnorm"] for x in st), "step_roofline_frac": sb / (ms / K / 1e3) / 1e9 / peak}
+               "divnorm_max": max(x["divnorm"] for x in st), "step_roofline_frac": per_s(step_bytes(S, n, st)),
+               "separate_pass_frac": per_s(separate_pass_bytes(S, n, sum(its) / len(its), c.pc_maxit))}
         sim.close()
         del sim
         torch.cuda.empty_cache()
@@ -369,7 +397,7 @@ def run_ours(args, rank, world, local):
     # overlap of consecutive kernels that the timed steps use
     sim.ctx.profile(True)
     sim.ctx.profile_read(reset=True)
-    timed(sim, args.steps)
+    stats_p = timed(sim, args.steps)[1]
     prof = sim.ctx.profile_read(reset=True)
     sim.ctx.profile(False)
     ms_max = max_over_ranks(ms, world)
@@ -377,23 +405,28 @@ def run_ours(args, rank, world, local):
     its = [s["it"] for s in stats]
     mean_it = sum(its) / len(its)
     value = replica_rate(world, n, args.steps, ms_max)
-    # dominant kernel class by device time
+    # dominant kernel class by device time; its launches with work (kernels queued
+    # after a pass has stopped return at once)
     cls = max((k for k in prof if k in KERNEL_VALUES), key=lambda k: prof[k][0])
-    tms, tn = prof[cls]
-    avg_ms = tms / max(tn, 1)
-    alg_bytes = KERNEL_VALUES[cls] * S * n
+    count = class_launches(stats_p, S == 4)
+    parts = [k for k in (cls, cls + "_first", cls + "_pass") if count.get(k)]
+    tn = sum(count[k] for k in parts)
+    avg_ms = prof[cls][0] / tn
+    alg_bytes = S * n * sum(KERNEL_VALUES[k] * count[k] for k in parts) / tn
     achieved = alg_bytes / (avg_ms / 1e3) / 1e9
-    step_b = step_bytes(S, n, mean_it)
+    step_b = step_bytes(S, n, stats)
+    sep_b = separate_pass_bytes(S, n, mean_it, case.pc_maxit)
     divmax = max(s["divnorm"] for s in stats)
     out.update({
         "value": value, "ms_per_step": ms_max / args.steps, "steps_per_s": 1e3 * args.steps / ms_max,
         "launches": launches, "its": it_summary(its), "divnorm_max": divmax, "div_ok": divmax <= 1e-6,
         "err_max": max(s["err"] for s in stats), "clocks": clk,
         "roofline": {"bound": "hbm", "kernel": cls, "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic_for(cls), "peak_kind": peak_kind,
+                     "frac": achieved / peak, "traffic": class_traffic(cls, count, S, n), "peak_kind": peak_kind,
                      "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms},
         "step_roofline": {"bytes_per_step": step_b, "achieved": step_b / (ms_max / args.steps / 1e3) / 1e9,
-                          "frac": step_b / (ms_max / args.steps / 1e3) / 1e9 / peak, "it": mean_it, "m": case.pc_maxit},
+                          "frac": step_b / (ms_max / args.steps / 1e3) / 1e9 / peak, "it": mean_it, "m": case.pc_maxit,
+                          "separate_pass_bytes": sep_b, "separate_pass_frac": sep_b / (ms_max / args.steps / 1e3) / 1e9 / peak},
         "profile": {k: {"ms": v[0], "launches": v[1]} for k, v in prof.items() if v[1]},
         "wall_s": wall,
     })

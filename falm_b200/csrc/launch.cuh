@@ -314,8 +314,14 @@ int sor_rb2_launch(falm_ctx *ctx, cudaStream_t st, const T *xin, const T *b, T *
 // whether three half sweeps run on the 28 x 16 skewed kernel rather than the
 // 32 x 8 one: always in FP32; in FP64 (2 CTAs per SM instead of 3) once every
 // CTA slot marches at least 128 planes, where its single barrier per plane
-// outweighs its longer pipeline fill (512x256x256: 0.725 -> 0.631 ms per pass;
-// 256x128x128, 35 planes per slot: 0.076 -> 0.083 ms)
+// outweighs its longer pipeline fill.  It is reached with three sweeps and more
+// (two run as half iterations, or on grids where neither kernel does).  FP64, us per
+// application of three / five sweeps, 32 x 8 and skewed: 128 x 64 x 64 45 and 48 /
+// 75 and 84, 256 x 128 x 128 187 and 198 / 312 and 335, 320 x 160 x 160 341 and 331 /
+// 570 and 528, 384 x 192 x 192 522 and 513 / 873 and 833, 448 x 224 x 224 830 and 750 /
+// 1395 and 1137, 512 x 256 x 256 1192 and 1144 / 1997 and 1840.  The line lies
+// between 384 x 192 x 192 and 448 x 224 x 224: below it the two are within 6% at three
+// sweeps; at five the skewed one would win from 320 x 160 x 160 on.
 template <typename T>
 bool sor_skewed(const falm_ctx *ctx) {
     if (ctx->sor_v1) return ctx->sor_v1 == 2;

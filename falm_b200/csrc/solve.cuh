@@ -78,9 +78,9 @@ int plain_solve_t(falm_ctx *ctx, T *x, const T *b, T *r, cudaStream_t st, int *i
 // (vectors, element type, whether the first preconditioner sweep is ready) and
 // dropped when the solver settings or the operator change.  Used by default
 // (FALM_B200_GRAPH=0 turns it off), never while profiling or checking launches
-// one by one: the unconditional iteration 1 and the condition kernels cost
-// less than the host round trips they replace, even at 1-2 iterations per
-// step on the 512x256x256 grid.
+// one by one: the unconditional iteration 1, whose kernels return at once when
+// the first converged, costs less than the host round trips it replaces, even at
+// 1-2 iterations per step on the 512x256x256 grid.
 constexpr int kMixedPassIts = 50;   // FP32 BiCGStab iterations between FP64 true-residual checks
 constexpr size_t kMaxRecordings = 16;   // recorded solves (and steps) kept per context
 

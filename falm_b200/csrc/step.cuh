@@ -88,7 +88,7 @@ int alm_run_t(falm_ctx *ctx, const T *u, T *ff, double t, cudaStream_t st, const
         const Region3 R = interior(ctx->geo);
         LAUNCH(FALM_K_ALM, st, k_alm_project<T><<<row_grid(ctx, R), kRowThreads, 0, st>>>(ctx->geo, R, mview<T>(ctx), mview<double>(ctx), ctx->alm, ff));
     } else if (ctx->alm.bs.total > 0) {
-        // force boxes for the fused projection of the plane-streaming pseudo-velocity kernel
+        // the force boxes, added by k_alm_add in a step and read by the plane-streaming pseudo-velocity kernel in falm_cfd_pseudo_u
         const long long blocks = std::min<long long>((ctx->alm.bs.total + 255) / 256, (long long)ctx->sm_count * 8);
         LAUNCH(FALM_K_ALM, st, k_alm_box<T><<<(int)blocks, 256, 0, st>>>(ctx->alm, ctx->m64.x[0], ctx->m64.x[1], ctx->m64.x[2]));
     }
